@@ -671,6 +671,8 @@ struct rgf_ctx {
   rgf_stats stats;
   int8_t variant[kVariantSlots];  // kernel variant per block size (defaults; rgf_autotune may override)
   int8_t ctas[kVariantSlots];     // resident CTAs per SM per block size, 0 = as many as fit
+  DevBuf scratch;                 // ctx_scratch, on CUDA device scratch_dev
+  int scratch_dev = -1;
   void* ext_cache = nullptr;      // per-context state of other modules (the FFT form's plans)
   void (*ext_cache_free)(void*) = nullptr;
   // pipelined host outputs (rgf_opts.pipelined): two staging slots used in
@@ -694,6 +696,15 @@ struct rgf_ctx {
   cudaEvent_t sync_solved = nullptr;
 };
 
+bool rgf::ctx_scratch(rgf_ctx* c, size_t bytes, void** p) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  if (dev != c->scratch_dev) c->scratch.release();
+  c->scratch_dev = dev;
+  if (c->scratch.reserve(bytes)) return false;
+  *p = c->scratch.p;
+  return true;
+}
 void* rgf::ctx_ext_cache(rgf_ctx* c) { return c->ext_cache; }
 void rgf::ctx_set_ext_cache(rgf_ctx* c, void* cache, void (*free_fn)(void*)) {
   c->ext_cache = cache;
@@ -782,6 +793,7 @@ extern "C" int rgf_ctx_destroy(rgf_ctx* c) {
   c->info.release();
   c->queue.release();
   c->stage.release();
+  c->scratch.release();
   if (c->stream) cudaStreamDestroy(c->stream);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);

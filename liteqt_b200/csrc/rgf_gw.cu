@@ -11,17 +11,15 @@
 // followed for S by the reference's Sigma^R imaginary part from
 // Sigma^> - Sigma^<, symmetrisation, mixing into the running self-energies
 // and the edge-block copies.  These are direct sums, as in the reference:
-// every output element is accumulated by one thread in the reference's
-// order (P: k then E; S: w then q).  Layout (nm,nm,nx,nen,nk) column-major,
-// k = kz + ky*nkz.
+// every output element is accumulated by one thread in a
+// fixed order (P: k then E; S: q then w).  Layout (nm,nm,nx,nen,nk) column-major, k = kz + ky*nkz.
 //
-// Memory pattern: when an element's energy series fit in shared memory
-// (6 nen complex values for P, 6 nen nk for S, up to 200 KB) a CTA stages
-// them once and sums from shared memory (the *_staged kernels); otherwise
-// the direct kernels have a warp take 32 consecutive energy offsets w (P) or
-// energies E (S) of one element, so one operand is the same address across
-// the warp and the other slides along the energy axis.
+// Three passes: the banded elements are gathered into series contiguous in
+// energy, the sums run on those with R outputs a thread in registers, and a
+// scatter pass writes the caller's arrays (for S with the post-processing).
+#include <algorithm>
 #include <cstdio>
+#include <type_traits>
 
 #include "rgf_device.cuh"
 #include "rgf_internal.h"
@@ -29,7 +27,6 @@
 namespace {
 
 constexpr double kPiGW = 3.14159265359;  // green_rgf.f90:23
-constexpr int kGWThreads = 128;
 
 struct GWDims {
   int64_t nm, nx, nen, nky, nkz, ndiag, nopmax;
@@ -52,6 +49,13 @@ struct GWDims {
   }
 };
 
+struct Arrays3 {          // three arrays in the caller's layout
+  const double2* a[3];
+};
+struct Lines3 {           // the same as lines (double or double2 values)
+  void* a[3];
+};
+
 __device__ __forceinline__ double2 gread(const double2* G, size_t k, int imag_only) {
   const double2 v = G[k];
   return imag_only ? make_double2(0.0 * v.x, v.y) : v;
@@ -60,20 +64,24 @@ __device__ __forceinline__ double2 gread(const double2* G, size_t k, int imag_on
 __device__ __forceinline__ double2 cfma(double2 acc, double2 a, double2 b) {
   return rgf::cadd(acc, rgf::cmul(a, b));
 }
+// acc += a b; a double stands for the imaginary number i a
+__device__ __forceinline__ void cfma_to(double2& acc, double2 a, double2 b) {
+  acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
+  acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));
+}
+__device__ __forceinline__ void cfma_to(double2& acc, double a, double2 b) {
+  acc.x = fma(-a, b.y, acc.x);
+  acc.y = fma(a, b.x, acc.y);
+}
 
-// grid: x = chunks of energy offsets, y = band element (i, jb), z = ix + nx*iq
-__global__ void __launch_bounds__(kGWThreads) gw_p_kernel(GWDims d, int imag_only, double2 scale,
-                                                           const double2* GL, const double2* GG,
-                                                           const double2* GR, double2* PL, double2* PG,
-                                                           double2* PR) {
-  const int64_t nop = -d.nopmax + (int64_t)blockIdx.x * kGWThreads + threadIdx.x;
-  if (nop > d.nopmax) return;
-  const int64_t i = blockIdx.y % d.nm, jb = blockIdx.y / d.nm;
-  const int64_t j = i - d.ndiag + jb;
-  if (j < 0 || j >= d.nm) return;
-  const int64_t ix = blockIdx.z % d.nx, iq = blockIdx.z / d.nx;
+// One output of the polarization, summed in the reference's own order and
+// with its complex products (k, then E).  The tiled kernels use it for lines
+// that hold an infinity or a NaN, where leaving a term out is not the same as
+// adding a zero.
+__device__ __noinline__ void p_reference_sum(const GWDims& d, int imag_only, int64_t nop, int64_t i, int64_t j,
+                                             int64_t ix, int64_t iq, Arrays3 G, double2 out[3]) {
+  const double2 *GL = G.a[0], *GG = G.a[1], *GR = G.a[2];
   const int64_t nk = d.nky * d.nkz;
-  const int64_t iop = nop + d.nen / 2 - 1;            // 0-based energy index of w
   double2 al = rgf::czero(), ag = rgf::czero(), ar = rgf::czero();
   const int64_t lo = (nop + 1 > 1 ? nop + 1 : 1) - 1;  // 0-based E range [lo, hi)
   const int64_t hi = d.nen < d.nen + nop ? d.nen : d.nen + nop;
@@ -90,24 +98,15 @@ __global__ void __launch_bounds__(kGWThreads) gw_p_kernel(GWDims d, int imag_onl
       ar = rgf::cadd(ar, rgf::cadd(rgf::cmul(gl, rgf::cconj(gread(GR, b, imag_only))), rgf::cmul(gr, glt)));
     }
   }
-  const size_t o = d.at(i, j, ix, iop, iq);
-  PL[o] = rgf::cmul(al, scale);
-  PG[o] = rgf::cmul(ag, scale);
-  PR[o] = rgf::cmul(ar, scale);
+  out[0] = al;
+  out[1] = ag;
+  out[2] = ar;
 }
 
-// grid: x = chunks of energies, y = band element (i, jb), z = ix + nx*ik
-__global__ void __launch_bounds__(kGWThreads) gw_s_kernel(GWDims d, int imag_only, double2 scale,
-                                                           const double2* GL, const double2* GG,
-                                                           const double2* GR, const double2* WL,
-                                                           const double2* WG, const double2* WR,
-                                                           double2* NL, double2* NG, double2* NR) {
-  const int64_t ie1 = (int64_t)blockIdx.x * kGWThreads + threadIdx.x + 1;  // 1-based E index
-  if (ie1 > d.nen) return;
-  const int64_t i = blockIdx.y % d.nm, jb = blockIdx.y / d.nm;
-  const int64_t j = i - d.ndiag + jb;
-  if (j < 0 || j >= d.nm) return;
-  const int64_t ix = blockIdx.z % d.nx, ik = blockIdx.z / d.nx;
+// One output of the self-energy in the reference's order (w, then q).
+__device__ __noinline__ void s_reference_sum(const GWDims& d, int imag_only, int64_t ie1, int64_t i, int64_t j,
+                                             int64_t ix, int64_t ik, Arrays3 G, Arrays3 W, double2 out[3]) {
+  const double2 *GL = G.a[0], *GG = G.a[1], *GR = G.a[2], *WL = W.a[0], *WG = W.a[1], *WR = W.a[2];
   const int64_t nk = d.nky * d.nkz;
   double2 al = rgf::czero(), ag = rgf::czero(), ar = rgf::czero();
   for (int64_t nop = -d.nopmax; nop <= d.nopmax; nop++) {
@@ -123,177 +122,416 @@ __global__ void __launch_bounds__(kGWThreads) gw_s_kernel(GWDims d, int imag_onl
       ar = rgf::cadd(ar, rgf::cadd(rgf::cadd(rgf::cmul(gl, wr), rgf::cmul(gr, wl)), rgf::cmul(gr, wr)));
     }
   }
-  const size_t o = d.at(i, j, ix, ie1 - 1, ik);
-  NL[o] = rgf::cmul(al, scale);
-  NG[o] = rgf::cmul(ag, scale);
-  NR[o] = rgf::cmul(ar, scale);
+  out[0] = al;
+  out[1] = ag;
+  out[2] = ar;
 }
 
-// Shared-memory staged forms of the two sums, used when the staged energy
-// series fit: a CTA owns one banded element (i, j, ix) and one q (P) or k
-// (Sigma) and all its energy offsets / energies (NPT per thread).  The
-// operands that the direct kernels read scattered along the energy axis are
-// read once per CTA into shared memory; every output keeps the reference's
-// order of summation (P: k, then E; Sigma: w, then q).
-constexpr int kStThreads = 256;
+// ---------------------------------------------------------------- band lines
+// The sums run along energy, the arrays have energy at stride nm^2 nx, so the
+// banded elements are first gathered into "lines": series of one element
+// (i, j, ix), contiguous in energy, line = (ix - ix0) * slots + slot, slot =
+// i + nm (j - i + nd) (nd = min(ndiag, nm - 1), slots = nm (2 nd + 1); the
+// few slots whose j lies outside the block stay unused).  A lines array is
+// [line][k][energy].
+struct Lines {
+  int64_t nd, slots, ix0;
+  __host__ __device__ int64_t slot(int64_t i, int64_t j, int64_t nm) const { return i + nm * (j - i + nd); }
+};
 
-template <int NPT>
-__global__ void __launch_bounds__(kStThreads) gw_p_staged_kernel(GWDims d, int imag_only, double2 scale,
-                                                                  const double2* GL, const double2* GG,
-                                                                  const double2* GR, double2* PL, double2* PG,
-                                                                  double2* PR) {
-  extern __shared__ __align__(16) double2 sh[];
-  const int64_t nen = d.nen;
-  double2 *aL = sh, *aG = sh + nen, *aR = sh + 2 * nen, *bG = sh + 3 * nen, *bL = sh + 4 * nen,
-          *bR = sh + 5 * nen;
-  const int64_t i = blockIdx.x % d.nm, jb = blockIdx.x / d.nm;
-  const int64_t j = i - d.ndiag + jb;
-  if (j < 0 || j >= d.nm) return;                      // uniform over the CTA
-  const int64_t ix = blockIdx.y, iq = blockIdx.z;
-  const int64_t nk = d.nky * d.nkz;
-  double2 al[NPT], ag[NPT], ar[NPT];
-#pragma unroll
-  for (int c = 0; c < NPT; c++) al[c] = ag[c] = ar[c] = rgf::czero();
-  for (int64_t ik = 0; ik < nk; ik++) {
-    const int64_t ikd = d.kd(ik, iq);
-    __syncthreads();
-    for (int64_t e = threadIdx.x; e < nen; e += kStThreads) {
-      const size_t a = d.at(i, j, ix, e, ik), bt = d.at(j, i, ix, e, ikd), b = d.at(i, j, ix, e, ikd);
-      aL[e] = gread(GL, a, imag_only);
-      aG[e] = gread(GG, a, imag_only);
-      aR[e] = gread(GR, a, imag_only);
-      bG[e] = gread(GG, bt, imag_only);
-      bL[e] = gread(GL, bt, imag_only);
-      bR[e] = gread(GR, b, imag_only);
+constexpr int kPackP = 64, kPackE = 32;   // elements x energies of a gather tile
+
+
+// Gathers three arrays into lines: the imaginary parts (IMAG) or the whole
+// values.  A CTA takes kPackP consecutive elements of the block x kPackE
+// energies of one (ix, k), so it reads contiguous runs and writes runs along
+// energy through shared memory.  flags[line] is set when a line holds an
+// infinity or a NaN.
+template <bool IMAG>
+__global__ void __launch_bounds__(256) gw_pack_kernel(GWDims d, Lines L, Arrays3 src, Lines3 dst,
+                                                       int* __restrict__ flags) {
+  using T = std::conditional_t<IMAG, double, double2>;
+  __shared__ T tile[kPackP][kPackE + 1];
+  const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
+  const int64_t p0 = (int64_t)blockIdx.x * kPackP, e0 = (int64_t)blockIdx.y * kPackE;
+  const int64_t ik = blockIdx.z % nk, ixl = blockIdx.z / nk;
+  auto band = [&](int64_t p, int64_t& slot) {
+    if (p >= n2) return false;
+    const int64_t i = p % d.nm, j = p / d.nm;
+    slot = L.slot(i, j, d.nm);
+    return i - j <= L.nd && j - i <= L.nd;
+  };
+  int64_t slot;
+  const int lp = threadIdx.x % kPackP;
+  const bool mine = band(p0 + lp, slot);
+  if (!__syncthreads_or(mine)) return;
+  for (int v = 0; v < 3; v++) {
+    if (mine) {
+      bool bad = false;
+      for (int le = threadIdx.x / kPackP; le < kPackE; le += 256 / kPackP) {
+        const int64_t e = e0 + le;
+        if (e >= d.nen) break;
+        const double2 x = src.a[v][p0 + lp + n2 * ((L.ix0 + ixl) + d.nx * (e + d.nen * ik))];
+        bad |= !(isfinite(x.x) && isfinite(x.y));
+        if constexpr (IMAG) tile[lp][le] = x.y;
+        else tile[lp][le] = x;
+      }
+      if (bad) flags[ixl * L.slots + slot] = 1;
     }
     __syncthreads();
+    for (int q = threadIdx.x; q < kPackP * kPackE; q += 256) {
+      const int le = q % kPackE, pp = q / kPackE;
+      int64_t sl;
+      if (e0 + le < d.nen && band(p0 + pp, sl))
+        ((T*)dst.a[v])[((ixl * L.slots + sl) * nk + ik) * d.nen + e0 + le] = tile[pp][le];
+    }
+    __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------- sums
+// Both sums are correlations along energy: output n of a line is
+// sum_u x(u) v(u - n), v a series that slides by one per step and per output.
+// A thread owns R consecutive outputs; at step u it needs v(u - n) for its R
+// outputs, of which R - 1 were already used at the step before, so it keeps
+// them in registers (slot (u - r) mod R for output r) and loads one new value
+// per series and step.  x(u) is the same for the whole CTA (a broadcast
+// read).  Tiles of TILE outputs x kSteps steps are staged in shared memory,
+// whatever nen is; v's position is padded by one per R values, so the lanes'
+// reads (R apart) fall on distinct banks.  The bound is the FP64 pipe: per
+// step and thread 32 multiply-adds against 6-7 shared loads.  Series are
+// finite here (other lines take the reference sum), so values outside a
+// series are zeros in shared memory instead of conditions in the loop.
+// Measured (1 B200, 1965 MHz) at nk = 4, nen = 512, nx = 10, nm = 16,
+// ndiag = 3, imaginary G: P 7.7 -> 1.75 ms, Sigma 12.6 -> 1.75 ms (complex
+// products on values staged whole, one output a thread, before), i.e. 14 and
+// 17 TFLOP/s of real multiply-adds; gathers 0.17 ms, scatters 0.31 ms.
+constexpr int kSteps = 64;
+
+template <bool IMAG>
+struct GwCfg {
+  static constexpr int TILE = IMAG ? 512 : 256;        // outputs a CTA
+  static constexpr int RP = IMAG ? 8 : 4;              // outputs a thread, polarization
+  static constexpr int RS = 4;                         // self-energy
+  static constexpr int TP = TILE / RP, TS = TILE / RS;  // threads
+};
+
+template <int R>
+__device__ __forceinline__ constexpr int vpos(int t) { return t + t / R; }
+template <int R, int TILE>
+constexpr int vlen() { return kSteps + TILE + (kSteps + TILE) / R + 1; }
+
+// Adds a chunk's sums to the running ones and clears them: sums of kSteps
+// terms added up have a smaller rounding error than one chain over all
+// terms.  The running sums sit in shared memory (one column a thread), which
+// the chunk's 32 kSteps multiply-adds hide.
+template <int N, int NT>
+__device__ __forceinline__ void flush(double (&run)[N][NT], double* part) {
 #pragma unroll
-    for (int c = 0; c < NPT; c++) {
-      const int64_t nop = -d.nopmax + threadIdx.x + (int64_t)kStThreads * c;
-      if (nop > d.nopmax) continue;
-      const int64_t lo = (nop + 1 > 1 ? nop + 1 : 1) - 1;
-      const int64_t hi = d.nen < d.nen + nop ? d.nen : d.nen + nop;
-      for (int64_t ie = lo; ie < hi; ie++) {
-        const int64_t e2 = ie - nop;
-        const double2 gl = aL[ie], glt = bL[e2];
-        al[c] = cfma(al[c], gl, bG[e2]);
-        ag[c] = cfma(ag[c], aG[ie], glt);
-        ar[c] = rgf::cadd(ar[c], rgf::cadd(rgf::cmul(gl, rgf::cconj(bR[e2])), rgf::cmul(aR[ie], glt)));
+  for (int k = 0; k < N; k++) {
+    run[k][threadIdx.x] += part[k];
+    part[k] = 0.0;
+  }
+}
+
+// Polarization of one (line, q), outputs nop of tile blockIdx.x:
+//   P^<(n) = sum_k sum_e G^<(e, k) G^>t(e - n, k - q), and the two others.
+// With purely imaginary G every product is one real multiply-add.  G: the
+// lines of G^<, G^>, G^R; out: lines [line][q][energy of n].
+template <bool IMAG>
+__global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L, double2 scale, int imag_only,
+                                                               Arrays3 src, Lines3 G, Lines3 out,
+                                                               const int* __restrict__ flags) {
+  using T = std::conditional_t<IMAG, double, double2>;
+  constexpr int R = GwCfg<IMAG>::RP, NT = GwCfg<IMAG>::TP, kTile = GwCfg<IMAG>::TILE;
+  constexpr int V = IMAG ? 1 : 2;                      // doubles per value
+  __shared__ T xs[3][kSteps];
+  __shared__ T vs[3][vlen<R, kTile>()];
+  __shared__ double run[3 * R * V][NT];
+  const int64_t nk = d.nky * d.nkz, nen = d.nen;
+  const int64_t slot = blockIdx.y, i = slot % d.nm, j = i - L.nd + slot / d.nm;
+  if (j < 0 || j >= d.nm) return;                      // uniform over the CTA
+  const int64_t iq = blockIdx.z % nk, ixl = blockIdx.z / nk;
+  const int64_t line = ixl * L.slots + slot, lineT = ixl * L.slots + L.slot(j, i, d.nm);
+  const int64_t n0 = -d.nopmax + (int64_t)blockIdx.x * kTile;
+  const int tid = threadIdx.x, q0 = R * tid;
+  const size_t orow = (size_t)(line * nk + iq) * nen + nen / 2 - 1;
+  if (flags[line] | flags[lineT]) {
+    for (int r = 0; r < R; r++) {
+      const int64_t nop = n0 + q0 + r;
+      if (nop > d.nopmax) break;
+      double2 a[3];
+      p_reference_sum(d, imag_only, nop, i, j, L.ix0 + ixl, iq, src, a);
+      for (int v = 0; v < 3; v++) ((double2*)out.a[v])[orow + nop] = rgf::cmul(a[v], scale);
+    }
+    return;
+  }
+  T acc[3][R];
+  T (&al)[R] = acc[0], (&ag)[R] = acc[1], (&ar)[R] = acc[2];
+#pragma unroll
+  for (int r = 0; r < R; r++) al[r] = ag[r] = ar[r] = T{};
+#pragma unroll
+  for (int k = 0; k < 3 * R * V; k++) run[k][tid] = 0.0;
+  // Imaginary G, n = 0, diagonal element: P^R is a difference of equal sums
+  // (of equal products where k - q = k), i.e. zero or the rounding of the
+  // reference's order.  The thread that owns that output forms it in that
+  // order, product by product, beside the chains of multiply-adds.
+  const bool owner = IMAG && i == j && n0 + q0 <= 0 && n0 + q0 + R > 0;
+  const int rz = (int)(-n0) - q0;
+  double pr0 = 0.0;
+  for (int64_t ik = 0; ik < nk; ik++) {
+    const size_t xrow = (size_t)(line * nk + ik) * nen;
+    const size_t vrow = (size_t)(line * nk + d.kd(ik, iq)) * nen, vrowT = (size_t)(lineT * nk + d.kd(ik, iq)) * nen;
+    for (int64_t e0 = 0; e0 < nen; e0 += kSteps) {
+      const int64_t vb = e0 - n0 - (kTile - 1);        // energy of position 0 of the sliding series
+      if (vb >= nen || vb + kTile - 1 + kSteps <= 0) continue;
+      __syncthreads();
+      for (int t = tid; t < kSteps; t += NT)
+#pragma unroll
+        for (int v = 0; v < 3; v++) xs[v][t] = e0 + t < nen ? ((const T*)G.a[v])[xrow + e0 + t] : T{};
+      for (int t = tid; t < kTile - 1 + kSteps; t += NT) {
+        const bool in = vb + t >= 0 && vb + t < nen;
+        vs[0][vpos<R>(t)] = in ? ((const T*)G.a[1])[vrowT + vb + t] : T{};   // G^>t
+        vs[1][vpos<R>(t)] = in ? ((const T*)G.a[0])[vrowT + vb + t] : T{};   // G^<t
+        vs[2][vpos<R>(t)] = in ? ((const T*)G.a[2])[vrow + vb + t] : T{};    // G^R
+      }
+      __syncthreads();
+      T w0[R], w1[R], w2[R];
+#pragma unroll
+      for (int r = 1; r < R; r++) {
+        const int p = vpos<R>(kTile - 1 - q0 - r);
+        w0[(R - r) % R] = vs[0][p];
+        w1[(R - r) % R] = vs[1][p];
+        w2[(R - r) % R] = vs[2][p];
+      }
+#pragma unroll 1
+      for (int u0 = 0; u0 < kSteps; u0 += R) {
+#pragma unroll
+        for (int c = 0; c < R; c++) {
+          const int p = vpos<R>(u0 + c + kTile - 1 - q0);
+          w0[c] = vs[0][p];
+          w1[c] = vs[1][p];
+          w2[c] = vs[2][p];
+          const T xl = xs[0][u0 + c], xg = xs[1][u0 + c], xr = xs[2][u0 + c];
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const int m = (c - r + R) % R;
+            if constexpr (IMAG) {
+              al[r] = fma(-xl, w0[m], al[r]);          // (i a)(i b) = -a b
+              ag[r] = fma(-xg, w1[m], ag[r]);
+              ar[r] = fma(xl, w2[m], fma(-xr, w1[m], ar[r]));
+            } else {
+              cfma_to(al[r], xl, w0[m]);
+              cfma_to(ag[r], xg, w1[m]);
+              cfma_to(ar[r], xl, rgf::cconj(w2[m]));
+              cfma_to(ar[r], xr, w1[m]);
+            }
+          }
+        }
+      }
+      flush(run, reinterpret_cast<double*>(acc));
+      if constexpr (IMAG) {
+        if (owner)
+#pragma unroll 4
+          for (int u = 0; u < kSteps; u++) {
+            const int p = vpos<R>(u + kTile - 1 - q0 - rz);
+            pr0 += __dsub_rn(__dmul_rn(xs[0][u], vs[2][p]), __dmul_rn(xs[2][u], vs[1][p]));
+          }
       }
     }
   }
 #pragma unroll
-  for (int c = 0; c < NPT; c++) {
-    const int64_t nop = -d.nopmax + threadIdx.x + (int64_t)kStThreads * c;
-    if (nop > d.nopmax) continue;
-    const size_t o = d.at(i, j, ix, nop + d.nen / 2 - 1, iq);
-    PL[o] = rgf::cmul(al[c], scale);
-    PG[o] = rgf::cmul(ag[c], scale);
-    PR[o] = rgf::cmul(ar[c], scale);
+  for (int r = 0; r < R; r++) {
+    const int64_t nop = n0 + q0 + r;
+    if (nop > d.nopmax) break;
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+      double2 z = make_double2(run[(v * R + r) * V][tid], IMAG ? 0.0 : run[(v * R + r) * V + V - 1][tid]);
+      if (IMAG && v == 2 && owner && r == rz) z.x = pr0;
+      ((double2*)out.a[v])[orow + nop] = rgf::cmul(z, scale);
+    }
   }
 }
 
-template <int NPT>
-__global__ void __launch_bounds__(kStThreads) gw_s_staged_kernel(GWDims d, int imag_only, double2 scale,
-                                                                  const double2* GL, const double2* GG,
-                                                                  const double2* GR, const double2* WL,
-                                                                  const double2* WG, const double2* WR,
-                                                                  double2* NL, double2* NG, double2* NR) {
-  extern __shared__ __align__(16) double2 sh[];
-  const int64_t nen = d.nen, nk = d.nky * d.nkz, ne = nen * nk;
-  double2 *gL = sh, *gG = sh + ne, *gR = sh + 2 * ne, *wL = sh + 3 * ne, *wG = sh + 4 * ne, *wR = sh + 5 * ne;
-  const int64_t i = blockIdx.x % d.nm, jb = blockIdx.x / d.nm;
-  const int64_t j = i - d.ndiag + jb;
+// Self-energy of one (line, k), energies of tile blockIdx.x:
+//   S^<(E) = sum_q sum_n G^<(E - n, k - q) W^<(n, q), and the two others;
+// G^R W^< + G^R W^R is formed as G^R (W^< + W^R).  The sums leave out the
+// first output energy and G's last one, as the reference's do (:3034).
+template <bool IMAG>
+__global__ void __launch_bounds__(GwCfg<IMAG>::TS) gw_s_kernel(GWDims d, Lines L, double2 scale, int imag_only,
+                                                               Arrays3 gsrc, Arrays3 wsrc, Lines3 G, Lines3 W,
+                                                               Lines3 out, const int* __restrict__ gflags,
+                                                               const int* __restrict__ wflags) {
+  using T = std::conditional_t<IMAG, double, double2>;
+  constexpr int R = GwCfg<IMAG>::RS, NT = GwCfg<IMAG>::TS, kTile = GwCfg<IMAG>::TILE;
+  __shared__ double2 xs[4][kSteps];                    // W^<, W^>, W^R, W^< + W^R
+  __shared__ T vs[3][vlen<R, kTile>()];
+  __shared__ double run[6 * R][NT];
+  const int64_t nk = d.nky * d.nkz, nen = d.nen, h = nen / 2 - 1;
+  const int64_t slot = blockIdx.y, i = slot % d.nm, j = i - L.nd + slot / d.nm;
   if (j < 0 || j >= d.nm) return;
-  const int64_t ix = blockIdx.y, ik = blockIdx.z;
-  // g(e, q) = G(i,j,ix,e,k-q), w(e, q) = W(i,j,ix,e,q) for every q
-  for (int64_t t = threadIdx.x; t < ne; t += kStThreads) {
-    const int64_t e = t % nen, iq = t / nen;
-    const size_t g = d.at(i, j, ix, e, d.kd(ik, iq)), w = d.at(i, j, ix, e, iq);
-    gL[t] = gread(GL, g, imag_only);
-    gG[t] = gread(GG, g, imag_only);
-    gR[t] = gread(GR, g, imag_only);
-    wL[t] = WL[w];
-    wG[t] = WG[w];
-    wR[t] = WR[w];
+  const int64_t ik = blockIdx.z % nk, ixl = blockIdx.z / nk;
+  const int64_t line = ixl * L.slots + slot;
+  const int64_t t0 = (int64_t)blockIdx.x * kTile;      // first energy of the tile
+  const int tid = threadIdx.x, q0 = R * tid;
+  const size_t orow = (size_t)(line * nk + ik) * nen;
+  if (gflags[line] | wflags[line]) {
+    for (int r = 0; r < R; r++) {
+      const int64_t e = t0 + q0 + r;
+      if (e >= nen) break;
+      double2 a[3];
+      s_reference_sum(d, imag_only, e + 1, i, j, L.ix0 + ixl, ik, gsrc, wsrc, a);
+      for (int v = 0; v < 3; v++) ((double2*)out.a[v])[orow + e] = rgf::cmul(a[v], scale);
+    }
+    return;
+  }
+  double2 acc[3][R];
+  double2 (&al)[R] = acc[0], (&ag)[R] = acc[1], (&ar)[R] = acc[2];
+#pragma unroll
+  for (int r = 0; r < R; r++) al[r] = ag[r] = ar[r] = rgf::czero();
+#pragma unroll
+  for (int k = 0; k < 6 * R; k++) run[k][tid] = 0.0;
+  for (int64_t iq = 0; iq < nk; iq++) {
+    const size_t wrow = (size_t)(line * nk + iq) * nen + h, grow = (size_t)(line * nk + d.kd(ik, iq)) * nen;
+    for (int64_t c0 = -d.nopmax; c0 <= d.nopmax; c0 += kSteps) {
+      const int64_t vb = t0 - c0 + kTile - 1;          // G energy of position 0 (positions run down)
+      if (vb < 0 || vb - (kTile - 1 + kSteps) >= nen - 1) continue;
+      __syncthreads();
+      for (int t = tid; t < kSteps; t += NT) {
+        const bool in = c0 + t <= d.nopmax;
+        const double2 wl = in ? ((const double2*)W.a[0])[wrow + c0 + t] : rgf::czero();
+        const double2 wr = in ? ((const double2*)W.a[2])[wrow + c0 + t] : rgf::czero();
+        xs[0][t] = wl;
+        xs[1][t] = in ? ((const double2*)W.a[1])[wrow + c0 + t] : rgf::czero();
+        xs[2][t] = wr;
+        xs[3][t] = rgf::cadd(wl, wr);
+      }
+      for (int t = tid; t < kTile - 1 + kSteps; t += NT) {
+        const int64_t e = vb - t;
+        const bool in = e >= 0 && e < nen - 1;
+#pragma unroll
+        for (int v = 0; v < 3; v++) vs[v][vpos<R>(t)] = in ? ((const T*)G.a[v])[grow + e] : T{};
+      }
+      __syncthreads();
+      T w0[R], w1[R], w2[R];
+#pragma unroll
+      for (int r = 1; r < R; r++) {
+        const int p = vpos<R>(kTile - 1 - q0 - r);
+        w0[(R - r) % R] = vs[0][p];
+        w1[(R - r) % R] = vs[1][p];
+        w2[(R - r) % R] = vs[2][p];
+      }
+#pragma unroll 1
+      for (int u0 = 0; u0 < kSteps; u0 += R) {
+#pragma unroll
+        for (int c = 0; c < R; c++) {
+          const int p = vpos<R>(u0 + c + kTile - 1 - q0);
+          w0[c] = vs[0][p];
+          w1[c] = vs[1][p];
+          w2[c] = vs[2][p];
+          const double2 xl = xs[0][u0 + c], xg = xs[1][u0 + c], xr = xs[2][u0 + c], xt = xs[3][u0 + c];
+#pragma unroll
+          for (int r = 0; r < R; r++) {
+            const int m = (c - r + R) % R;
+            cfma_to(al[r], w0[m], xl);
+            cfma_to(ag[r], w1[m], xg);
+            cfma_to(ar[r], w0[m], xr);
+            cfma_to(ar[r], w2[m], xt);
+          }
+        }
+      }
+      flush(run, reinterpret_cast<double*>(acc));
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < R; r++) {
+    const int64_t e = t0 + q0 + r;
+    if (e >= nen) break;
+#pragma unroll
+    for (int v = 0; v < 3; v++) {
+      const double2 z = make_double2(run[2 * (v * R + r)][tid], run[2 * (v * R + r) + 1][tid]);
+      ((double2*)out.a[v])[orow + e] = e == 0 ? rgf::czero() : rgf::cmul(z, scale);
+    }
+  }
+}
+
+// ---------------------------------------------------------------- scatter
+constexpr int kOutP = 16, kOutE = 32;   // elements x energies of a scatter tile
+
+// P lines -> the caller's arrays, every element of the blocks ix0.. written:
+// zero outside the band and outside the window of energy offsets.
+__global__ void __launch_bounds__(256) gw_p_scatter_kernel(GWDims d, Lines L, Lines3 P, Lines3 out) {
+  __shared__ double2 tile[3][kOutP][kOutE + 1];
+  const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
+  const int64_t p0 = (int64_t)blockIdx.x * kOutP, e0 = (int64_t)blockIdx.y * kOutE;
+  const int64_t iq = blockIdx.z % nk, ixl = blockIdx.z / nk;
+  const int64_t lo = d.nen / 2 - 1 - d.nopmax, hi = d.nen / 2 - 1 + d.nopmax;
+  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+    const int le = q % kOutE, lp = q / kOutE;
+    const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
+    const bool in = p < n2 && i - j <= L.nd && j - i <= L.nd && e >= lo && e <= hi;
+#pragma unroll
+    for (int v = 0; v < 3; v++)
+      tile[v][lp][le] = in ? ((const double2*)P.a[v])[((ixl * L.slots + L.slot(i, j, d.nm)) * nk + iq) * d.nen + e]
+                           : rgf::czero();
   }
   __syncthreads();
-  double2 al[NPT], ag[NPT], ar[NPT];
+  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+    const int lp = q % kOutP, le = q / kOutP;
+    const int64_t p = p0 + lp, e = e0 + le;
+    if (p >= n2 || e >= d.nen) continue;
+    const size_t o = (size_t)p + (size_t)n2 * ((L.ix0 + ixl) + (size_t)d.nx * (e + (size_t)d.nen * iq));
 #pragma unroll
-  for (int c = 0; c < NPT; c++) al[c] = ag[c] = ar[c] = rgf::czero();
-  for (int64_t nop = -d.nopmax; nop <= d.nopmax; nop++) {
-    const int64_t iop = nop + nen / 2 - 1;
-    for (int64_t iq = 0; iq < nk; iq++) {
-      const double2 wl = wL[iop + nen * iq], wg = wG[iop + nen * iq], wr = wR[iop + nen * iq];
+    for (int v = 0; v < 3; v++) ((double2*)out.a[v])[o] = tile[v][lp][le];
+  }
+}
+
+// Sigma lines (N: S^<, S^>, S^R) -> the running self-energies: Sigma^R's
+// imaginary part from Sigma^> - Sigma^<, symmetrisation and mixing
+// (green_rgf.f90:3068-3085), then the edge-block copies (:3087-3092) in the
+// same pass: blocks 1, 2 repeat block 3 and blocks nx-1, nx block nx-2, so
+// only the blocks in between are summed and each writes its own copies.
+// have = false: the window of offsets is empty and every new value is zero.
+__global__ void __launch_bounds__(256) gw_s_scatter_kernel(GWDims d, Lines L, double alpha, bool have, Lines3 N,
+                                                           Lines3 S) {
+  __shared__ double2 tile[3][kOutP][kOutE + 1];
+  const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
+  const int64_t p0 = (int64_t)blockIdx.x * kOutP, e0 = (int64_t)blockIdx.y * kOutE;
+  const int64_t ik = blockIdx.z % nk, ixl = blockIdx.z / nk, ix = L.ix0 + ixl;
+  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+    const int le = q % kOutE, lp = q / kOutE;
+    const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
+    double2 nl = rgf::czero(), ng = nl, nr = nl;
+    if (have && p < n2 && i - j <= L.nd && j - i <= L.nd && e < d.nen) {
+      const size_t a = (size_t)((ixl * L.slots + L.slot(i, j, d.nm)) * nk + ik) * d.nen + e;
+      const size_t b = (size_t)((ixl * L.slots + L.slot(j, i, d.nm)) * nk + ik) * d.nen + e;
+      const double2 *NL = (const double2*)N.a[0], *NG = (const double2*)N.a[1], *NR = (const double2*)N.a[2];
+      const double2 la = NL[a], lb = NL[b], ga = NG[a], gb = NG[b];
+      auto sym = [](double2 x, double2 y) { return make_double2((x.x + y.x) / 2.0, (x.y + y.y) / 2.0); };
+      nr = sym(make_double2(NR[a].x, (ga.y - la.y) / 2.0), make_double2(NR[b].x, (gb.y - lb.y) / 2.0));
+      nl = sym(la, lb);
+      ng = sym(ga, gb);
+    }
+    tile[0][lp][le] = nl;
+    tile[1][lp][le] = ng;
+    tile[2][lp][le] = nr;
+  }
+  __syncthreads();
+  const bool all = d.nx < 5;                            // every block repeats block 3
+  const int64_t d0 = all ? 0 : (ix == 2 ? 0 : ix), d1 = all ? d.nx - 1 : (ix == d.nx - 3 ? d.nx - 1 : ix);
+  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+    const int lp = q % kOutP, le = q / kOutP;
+    const int64_t p = p0 + lp, e = e0 + le;
+    if (p >= n2 || e >= d.nen) continue;
+    const size_t row = (size_t)d.nx * (e + (size_t)d.nen * ik);
 #pragma unroll
-      for (int c = 0; c < NPT; c++) {
-        const int64_t ie1 = 1 + threadIdx.x + (int64_t)kStThreads * c;
-        if (ie1 > nen || !(ie1 > (nop > 1 ? nop : 1) && ie1 < nen + nop)) continue;
-        const int64_t g = ie1 - nop - 1 + nen * iq;
-        const double2 gl = gL[g], gr = gR[g];
-        al[c] = cfma(al[c], gl, wl);
-        ag[c] = cfma(ag[c], gG[g], wg);
-        ar[c] = rgf::cadd(ar[c], rgf::cadd(rgf::cadd(rgf::cmul(gl, wr), rgf::cmul(gr, wl)), rgf::cmul(gr, wr)));
-      }
+    for (int v = 0; v < 3; v++) {
+      double2* A = (double2*)S.a[v];
+      const double2 s = A[(size_t)p + (size_t)n2 * (ix + row)];
+      const double2 r = rgf::cadd(s, rgf::cscale(rgf::csub(tile[v][lp][le], s), alpha));
+      for (int64_t b = d0; b <= d1; b++) A[(size_t)p + (size_t)n2 * (b + row)] = r;
     }
   }
-#pragma unroll
-  for (int c = 0; c < NPT; c++) {
-    const int64_t ie1 = 1 + threadIdx.x + (int64_t)kStThreads * c;
-    if (ie1 > nen) continue;
-    const size_t o = d.at(i, j, ix, ie1 - 1, ik);
-    NL[o] = rgf::cmul(al[c], scale);
-    NG[o] = rgf::cmul(ag[c], scale);
-    NR[o] = rgf::cmul(ar[c], scale);
-  }
-}
-
-constexpr size_t kGWStagedSmemMax = 200 * 1024;
-
-// Launch a staged kernel with NPT = the smallest of 1, 2, 4, 8 covering
-// `count` values per CTA; false if none fits (the caller then uses the
-// direct kernel).
-template <class L1, class L2, class L4, class L8>
-bool launch_npt(int64_t count, size_t smem, L1 l1, L2 l2, L4 l4, L8 l8) {
-  if (smem > kGWStagedSmemMax) return false;
-  const int64_t npt = (count + kStThreads - 1) / kStThreads;
-  if (npt <= 1) l1(); else if (npt <= 2) l2(); else if (npt <= 4) l4(); else if (npt <= 8) l8(); else return false;
-  return true;
-}
-
-// Sigma^R imaginary part from Sigma^> - Sigma^<, symmetrisation and mixing
-// (green_rgf.f90:3068-3085); one thread per element of the whole arrays.
-__global__ void gw_s_post_kernel(int64_t nm, int64_t total, double alpha, const double2* NL,
-                                 const double2* NG, const double2* NR, double2* SL, double2* SG,
-                                 double2* SR) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= total) return;
-  const int64_t n2 = nm * nm, blk = k / n2, r = k % n2, i = r % nm, j = r / nm;
-  const int64_t kt = blk * n2 + j + i * nm;
-  auto fixr = [&](int64_t q) { return make_double2(NR[q].x, (NG[q].y - NL[q].y) / 2.0); };
-  auto sym = [](double2 a, double2 b) { return make_double2((a.x + b.x) / 2.0, (a.y + b.y) / 2.0); };
-  const double2 nr = sym(fixr(k), fixr(kt)), nl = sym(NL[k], NL[kt]), ng = sym(NG[k], NG[kt]);
-  auto mix = [&](double2* S, double2 nv) {
-    const double2 s = S[k];
-    S[k] = rgf::cadd(s, rgf::cscale(rgf::csub(nv, s), alpha));
-  };
-  mix(SR, nr);
-  mix(SL, nl);
-  mix(SG, ng);
-}
-
-// A(:,:,dst,:,:) = A(:,:,src,:,:) for the three arrays (0-based blocks)
-__global__ void gw_copy_block_kernel(int64_t nm, int64_t nx, int64_t nsets, int64_t dst, int64_t src,
-                                     double2* A, double2* B, double2* C) {
-  const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t n2 = nm * nm;
-  if (k >= n2 * nsets) return;
-  const int64_t set = k / n2, r = k % n2;
-  const size_t s = (size_t)r + (size_t)n2 * (src + (size_t)nx * set);
-  const size_t t = (size_t)r + (size_t)n2 * (dst + (size_t)nx * set);
-  A[t] = A[s];
-  B[t] = B[s];
-  C[t] = C[s];
 }
 
 bool on_device(const void* p) {
@@ -335,6 +573,52 @@ int gw_fail(int code, const char* msg) {
   return code;
 }
 
+// Scratch of one call (the context's, kept between calls): the lines of as
+// many blocks ix as fit kWorkBytes, at least one, and a flag per line.  The
+// calls return with their stream drained, so the next one may reuse it.
+struct Workspace {
+  static constexpr size_t kWorkBytes = size_t(2) << 30;
+  int64_t nd = 0, slots = 0, nix = 0;
+  size_t per_line = 0;
+  char* base = nullptr;
+  int* flags = nullptr;
+
+  // bytes_per_value: of all the lines arrays together
+  int open(rgf_ctx* ctx, const GWDims& d, int64_t ix0, int64_t ix1, size_t bytes_per_value, int nflags) {
+    nd = std::min(d.ndiag, d.nm - 1);
+    slots = d.nm * (2 * nd + 1);
+    per_line = (size_t)d.nky * d.nkz * d.nen;
+    const size_t per_ix = (size_t)slots * per_line * bytes_per_value;
+    nix = std::max<int64_t>(1, std::min<int64_t>(ix1 - ix0, (int64_t)(kWorkBytes / per_ix)));
+    const size_t lines = (per_ix * nix + 255) & ~size_t(255);
+    void* p = nullptr;
+    if (!rgf::ctx_scratch(ctx, lines + sizeof(int) * (size_t)nflags * nix * slots, &p))
+      return gw_fail(RGF_E_NOMEM, "device scratch for the convolutions");
+    base = (char*)p;
+    flags = (int*)(base + lines);
+    return RGF_OK;
+  }
+  // three lines arrays of `val`-byte values for n blocks, after `before` bytes
+  // per value (the 16-byte ones first, which keeps them aligned)
+  Lines3 take(size_t val, int64_t n, size_t before) const {
+    const size_t len = (size_t)slots * n * per_line;
+    char* p = base + len * before;
+    return Lines3{{p, p + len * val, p + 2 * len * val}};
+  }
+  void pack(const GWDims& d, const Lines& L, int64_t n, bool imag, const Arrays3& src, const Lines3& dst, int* fl,
+            cudaStream_t st) const {
+    cudaMemsetAsync(fl, 0, sizeof(int) * (size_t)n * slots, st);
+    const dim3 grid((unsigned)((d.nm * d.nm + kPackP - 1) / kPackP), (unsigned)((d.nen + kPackE - 1) / kPackE),
+                    (unsigned)(n * d.nky * d.nkz));
+    if (imag) gw_pack_kernel<true><<<grid, 256, 0, st>>>(d, L, src, dst, fl);
+    else gw_pack_kernel<false><<<grid, 256, 0, st>>>(d, L, src, dst, fl);
+  }
+  dim3 out_grid(const GWDims& d, int64_t n) const {
+    return dim3((unsigned)((d.nm * d.nm + kOutP - 1) / kOutP), (unsigned)((d.nen + kOutE - 1) / kOutE),
+                (unsigned)(n * d.nky * d.nkz));
+  }
+};
+
 int check_dims(int64_t nm, int64_t nx, int64_t nen, int64_t nky, int64_t nkz, int64_t ndiag) {
   if (nm < 1 || nm > 4096 || nx < 3 || nen < 1 || nky < 1 || nkz < 1 || ndiag < 0)
     return gw_fail(RGF_E_ARG, "invalid GW dimensions (nx >= 3 for the edge-block copies)");
@@ -368,25 +652,26 @@ extern "C" int rgf_gw_polarization(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t
   if (e == cudaSuccess) e = pg.open(P_greater, bytes, false, true, st);
   if (e == cudaSuccess) e = pr.open(P_retarded, bytes, false, true, st);
   if (e != cudaSuccess) return gw_fail(RGF_E_CUDA, cudaGetErrorString(e));
-  for (View* v : {&pl, &pg, &pr}) cudaMemsetAsync(v->dev, 0, bytes, st);
   GWDims d{nm, nx, nen, nky, nkz, ndiag, nen / 2 - 10};
-  if (d.nopmax >= 0) {
+  if (d.nopmax < 0) {
+    for (View* v : {&pl, &pg, &pr}) cudaMemsetAsync(v->dev, 0, bytes, st);
+  } else {
     const double2 scale = make_double2(0.0, -1.0 * dE / 2.0 / kPiGW * spindeg / (double)nk);
-    const double2 *a = (const double2*)gl.dev, *b = (const double2*)gg.dev, *c = (const double2*)gr.dev;
-    double2 *o1 = (double2*)pl.dev, *o2 = (double2*)pg.dev, *o3 = (double2*)pr.dev;
-    const dim3 sgrid((unsigned)(nm * (2 * ndiag + 1)), (unsigned)nx, (unsigned)nk);
-    const size_t smem = 6 * sizeof(double2) * (size_t)nen;
-    auto go = [&](auto kern) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      kern<<<sgrid, kStThreads, smem, st>>>(d, imag_only, scale, a, b, c, o1, o2, o3);
-    };
-    const bool staged = launch_npt(
-        2 * d.nopmax + 1, smem, [&] { go(gw_p_staged_kernel<1>); }, [&] { go(gw_p_staged_kernel<2>); },
-        [&] { go(gw_p_staged_kernel<4>); }, [&] { go(gw_p_staged_kernel<8>); });
-    if (!staged) {
-      dim3 grid((unsigned)((2 * d.nopmax + 1 + kGWThreads - 1) / kGWThreads), (unsigned)(nm * (2 * ndiag + 1)),
-                (unsigned)(nx * nk));
-      gw_p_kernel<<<grid, kGWThreads, 0, st>>>(d, imag_only, scale, a, b, c, o1, o2, o3);
+    const Arrays3 G{{(const double2*)gl.dev, (const double2*)gg.dev, (const double2*)gr.dev}};
+    const Lines3 out{{pl.dev, pg.dev, pr.dev}};
+    const size_t val = imag_only ? sizeof(double) : sizeof(double2);
+    const int64_t tile = imag_only ? GwCfg<true>::TILE : GwCfg<false>::TILE;
+    Workspace ws;
+    if ((rc = ws.open(ctx, d, 0, nx, 3 * val + 3 * sizeof(double2), 1)) != RGF_OK) return rc;
+    for (int64_t ix0 = 0; ix0 < nx; ix0 += ws.nix) {
+      const int64_t n = std::min(ws.nix, nx - ix0);
+      const Lines L{ws.nd, ws.slots, ix0};
+      const Lines3 pp = ws.take(sizeof(double2), n, 0), gp = ws.take(val, n, 3 * sizeof(double2));
+      ws.pack(d, L, n, imag_only, G, gp, ws.flags, st);
+      const dim3 grid((unsigned)((2 * d.nopmax + tile) / tile), (unsigned)ws.slots, (unsigned)(n * nk));
+      if (imag_only) gw_p_kernel<true><<<grid, GwCfg<true>::TP, 0, st>>>(d, L, scale, imag_only, G, gp, pp, ws.flags);
+      else gw_p_kernel<false><<<grid, GwCfg<false>::TP, 0, st>>>(d, L, scale, imag_only, G, gp, pp, ws.flags);
+      gw_p_scatter_kernel<<<ws.out_grid(d, n), 256, 0, st>>>(d, L, pp, out);
     }
   }
   e = cudaGetLastError();
@@ -410,7 +695,7 @@ extern "C" int rgf_gw_self_energy(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t 
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nk = nky * nkz;
-  const size_t nel = (size_t)nm * nm * nx * nen * nk, bytes = sizeof(rgf_c16) * nel;
+  const size_t bytes = sizeof(rgf_c16) * (size_t)nm * nm * nx * nen * nk;
   View gl, gg, gr, wl, wg, wr, sl, sg, sr;
   cudaError_t e = gl.open((void*)G_lesser, bytes, true, false, st);
   if (e == cudaSuccess) e = gg.open((void*)G_greater, bytes, true, false, st);
@@ -421,48 +706,42 @@ extern "C" int rgf_gw_self_energy(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t 
   if (e == cudaSuccess) e = sl.open(Sigma_lesser_gw, bytes, true, true, st);
   if (e == cudaSuccess) e = sg.open(Sigma_greater_gw, bytes, true, true, st);
   if (e == cudaSuccess) e = sr.open(Sigma_r_gw, bytes, true, true, st);
-  double2* nbuf = nullptr;
-  if (e == cudaSuccess) e = cudaMalloc(&nbuf, 3 * bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return gw_fail(e == cudaErrorMemoryAllocation ? RGF_E_NOMEM : RGF_E_CUDA, cudaGetErrorString(e));
   }
-  cudaMemsetAsync(nbuf, 0, 3 * bytes, st);
-  double2 *NL = nbuf, *NG = nbuf + nel, *NR = nbuf + 2 * nel;
   GWDims d{nm, nx, nen, nky, nkz, ndiag, nen / 2 - 10};
-  if (d.nopmax >= 0) {
-    const double2 scale = make_double2(0.0, dE / 2.0 / kPiGW / (double)nk);
-    const double2 *a = (const double2*)gl.dev, *b = (const double2*)gg.dev, *c = (const double2*)gr.dev;
-    const double2 *w1 = (const double2*)wl.dev, *w2 = (const double2*)wg.dev, *w3 = (const double2*)wr.dev;
-    const dim3 sgrid((unsigned)(nm * (2 * ndiag + 1)), (unsigned)nx, (unsigned)nk);
-    const size_t smem = 6 * sizeof(double2) * (size_t)nen * (size_t)nk;
-    auto go = [&](auto kern) {
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      kern<<<sgrid, kStThreads, smem, st>>>(d, imag_only, scale, a, b, c, w1, w2, w3, NL, NG, NR);
-    };
-    const bool staged = launch_npt(
-        nen, smem, [&] { go(gw_s_staged_kernel<1>); }, [&] { go(gw_s_staged_kernel<2>); },
-        [&] { go(gw_s_staged_kernel<4>); }, [&] { go(gw_s_staged_kernel<8>); });
-    if (!staged) {
-      dim3 grid((unsigned)((nen + kGWThreads - 1) / kGWThreads), (unsigned)(nm * (2 * ndiag + 1)),
-                (unsigned)(nx * nk));
-      gw_s_kernel<<<grid, kGWThreads, 0, st>>>(d, imag_only, scale, a, b, c, w1, w2, w3, NL, NG, NR);
+  const bool have = d.nopmax >= 0;
+  const double2 scale = make_double2(0.0, dE / 2.0 / kPiGW / (double)nk);
+  const Arrays3 G{{(const double2*)gl.dev, (const double2*)gg.dev, (const double2*)gr.dev}};
+  const Arrays3 W{{(const double2*)wl.dev, (const double2*)wg.dev, (const double2*)wr.dev}};
+  const Lines3 S{{sl.dev, sg.dev, sr.dev}};
+  // the blocks that are summed: the edge copies overwrite the others
+  const int64_t first = 2, last = nx < 5 ? 2 : nx - 3;
+  const size_t val = imag_only ? sizeof(double) : sizeof(double2);
+  const int64_t tile = imag_only ? GwCfg<true>::TILE : GwCfg<false>::TILE;
+  Workspace ws;
+  if ((rc = ws.open(ctx, d, first, last + 1, 3 * val + 6 * sizeof(double2), 2)) != RGF_OK) return rc;
+  for (int64_t ix0 = first; ix0 <= last; ix0 += ws.nix) {
+    const int64_t n = std::min(ws.nix, last + 1 - ix0);
+    const Lines L{ws.nd, ws.slots, ix0};
+    const Lines3 wp = ws.take(sizeof(double2), n, 0), np = ws.take(sizeof(double2), n, 3 * sizeof(double2)),
+                 gp = ws.take(val, n, 6 * sizeof(double2));
+    if (have) {
+      int* wflags = ws.flags + ws.nix * ws.slots;
+      ws.pack(d, L, n, imag_only, G, gp, ws.flags, st);
+      ws.pack(d, L, n, false, W, wp, wflags, st);
+      const dim3 grid((unsigned)((nen + tile - 1) / tile), (unsigned)ws.slots, (unsigned)(n * nk));
+      if (imag_only)
+        gw_s_kernel<true><<<grid, GwCfg<true>::TS, 0, st>>>(d, L, scale, imag_only, G, W, gp, wp, np, ws.flags, wflags);
+      else
+        gw_s_kernel<false><<<grid, GwCfg<false>::TS, 0, st>>>(d, L, scale, imag_only, G, W, gp, wp, np, ws.flags, wflags);
     }
+    gw_s_scatter_kernel<<<ws.out_grid(d, n), 256, 0, st>>>(d, L, alpha_mix, have, np, S);
   }
-  const int tpb = 256;
-  gw_s_post_kernel<<<(unsigned)((nel + tpb - 1) / tpb), tpb, 0, st>>>(
-      nm, (int64_t)nel, alpha_mix, NL, NG, NR, (double2*)sl.dev, (double2*)sg.dev, (double2*)sr.dev);
-  // edge blocks (green_rgf.f90:3087-3092): 1, 2 <- 3, then nx, nx-1 <- nx-2
-  const int64_t nsets = nen * nk;
-  const unsigned cg = (unsigned)((nm * nm * nsets + tpb - 1) / tpb);
-  const int64_t copies[4][2] = {{0, 2}, {1, 2}, {nx - 1, nx - 3}, {nx - 2, nx - 3}};
-  for (const auto& c : copies)
-    gw_copy_block_kernel<<<cg, tpb, 0, st>>>(nm, nx, nsets, c[0], c[1], (double2*)sr.dev,
-                                             (double2*)sl.dev, (double2*)sg.dev);
   e = cudaGetLastError();
   for (View* v : {&sl, &sg, &sr})
     if (e == cudaSuccess) e = v->finish(st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-  cudaFree(nbuf);
   return e == cudaSuccess ? RGF_OK : gw_fail(RGF_E_CUDA, cudaGetErrorString(e));
 }
