@@ -16,9 +16,21 @@
 //   Sigma^(p) = G^(p) W^(p)  exp(+2 pi i p.s/nk) / (nk N) * dE_S
 // and one inverse 3-D FFT per output gives every q (or k) at once.  The
 // window read back is the 'fft' paths' one: P(p) at energy shift
-// b = p - 1 - n/2, Sigma(e) from W placed at nop = -(n/2-1) .. n/2-1.  The
-// FFTs are cuFFT's (Z2Z, batched, stream-ordered); packing, the frequency
-// products and the window extraction are kernels of this file.
+// b = p - 1 - n/2, Sigma(e) from W placed at nop = -(n/2-1) .. n/2-1.
+//
+// Up to nen = 4096 (N = 8192) the transforms are this library's own, and the
+// energy axis never leaves the SM between transform, product and inverse:
+//   k_forward   the k-grid transform of every operand (nen values a line and
+//               k, before any padding), one read and one write;
+//   line_*      per (line, k-frequency): the energy transforms of all operands
+//               one after another (registers + one shared buffer,
+//               rgf_fft_smem.cuh), the products, the inverse transforms and
+//               the window; spectra that wait for a partner go to scratch of
+//               the resident CTAs (L2);
+//   k_inverse   the inverse k-grid transform of the windows with the phases.
+// Longer axes and k-grids whose tile does not fit take the form below it:
+// cuFFT's 3-D transforms (Z2Z, batched, stream-ordered) with separate packing,
+// product and window kernels.
 //
 // Arrays: the *_by_blocks layout (nen, nk, nx, nij) complex(8) on the device,
 // energy fastest, ik = ikz + nkz (iky) (0-based).  nen must be even.
@@ -31,6 +43,7 @@
 #include <memory>
 #include <vector>
 
+#include "rgf_fft_smem.cuh"
 #include "rgf_internal.h"
 
 namespace {
@@ -151,6 +164,332 @@ __global__ void unpack_kernel(const double2* __restrict__ b0, const double2* __r
   }
 }
 
+// ------------------------------------------------------------ own transforms
+namespace own {
+
+using rgf::fft::add;
+using rgf::fft::mul;
+using rgf::fft::mulc;
+
+constexpr int kMinLog = 5, kMaxLog = 12;   // log2 of M, half the circular length
+
+// DFT of x[0], x[S], ... (L values), exp(-2 pi i) forward, + inverse.
+template <int L, int S, bool INV>
+__device__ __forceinline__ void dft_small(double2* x) {
+  if constexpr (L == 2) {
+    const double2 a = x[0], b = x[S];
+    x[0] = add(a, b);
+    x[S] = rgf::fft::sub(a, b);
+  } else if constexpr (L == 4) {
+    rgf::fft::dft4<INV>(x[0], x[S], x[2 * S], x[3 * S]);
+  }
+}
+
+template <int NKY, int NKZ, bool INV>
+__device__ __forceinline__ void dft_k(double2 (&x)[NKY * NKZ]) {
+#pragma unroll
+  for (int y = 0; y < NKY; y++) dft_small<NKZ, 1, INV>(x + y * NKZ);
+#pragma unroll
+  for (int z = 0; z < NKZ; z++) dft_small<NKY, NKZ, INV>(x + z);
+}
+
+struct Six {
+  const double2* a[6];
+};
+struct Three {
+  double2* a[3];
+};
+
+// k-grid transform of operand blockIdx.z of the lines of a chunk into
+// kb[op][line][k][energy]; bit op of `conj`: of its conjugate.  One thread an
+// energy with its nk values in registers: bound by one read and one write.
+template <int NKY, int NKZ>
+__global__ void __launch_bounds__(256) k_forward(Six in, const int64_t* __restrict__ lines, int64_t nl, Dims d,
+                                                 unsigned conj, double2* __restrict__ kb) {
+  constexpr int NK = NKY * NKZ;
+  const int op = blockIdx.z;
+  const int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x, b = blockIdx.y;
+  if (e >= d.nen) return;
+  const double2* src = in.a[op] + lines[b] * NK * d.nen + e;
+  double2* dst = kb + ((size_t)op * nl + b) * NK * d.nen + e;
+  const double sg = (conj >> op) & 1 ? -1.0 : 1.0;
+  double2 x[NK];
+#pragma unroll
+  for (int k = 0; k < NK; k++) {
+    const double2 v = src[k * d.nen];
+    x[k] = make_double2(v.x, sg * v.y);
+  }
+  dft_k<NKY, NKZ, false>(x);
+#pragma unroll
+  for (int k = 0; k < NK; k++) dst[k * d.nen] = x[k];
+}
+
+// Windows pb[v][line][k-frequency][energy] times ph -> outputs of the lines.
+// fix: Sigma^R's imaginary part is (Im Sigma^> - Im Sigma^<) / 2.
+template <int NKY, int NKZ>
+__global__ void __launch_bounds__(128) k_inverse(Three out, const int64_t* __restrict__ lines, int64_t nl, Dims d,
+                                                 bool fix, const double2* __restrict__ ph,
+                                                 const double2* __restrict__ pb) {
+  constexpr int NK = NKY * NKZ;
+  const int64_t e = (int64_t)blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
+  if (e >= d.nen) return;
+  double diff[NK];
+#pragma unroll
+  for (int k = 0; k < NK; k++) diff[k] = 0.0;
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    const double2* src = pb + ((size_t)v * nl + b) * NK * d.nen + e;
+    double2* dst = out.a[v] + lines[b] * NK * d.nen + e;
+    double2 x[NK];
+#pragma unroll
+    for (int k = 0; k < NK; k++) x[k] = mul(src[k * d.nen], ph[k]);
+    dft_k<NKY, NKZ, true>(x);
+#pragma unroll
+    for (int k = 0; k < NK; k++) {
+      if (v == 0) diff[k] = -x[k].y;
+      else if (v == 1) diff[k] += x[k].y;
+      else if (fix) x[k].y = diff[k] / 2.0;
+      dst[k * d.nen] = x[k];
+    }
+  }
+}
+
+// The same two for any k-grid: a tile of 32 energies in shared memory, the
+// two axes one after another as sums over the axis (tables of the nky-th and
+// nkz-th roots behind the ph table).
+constexpr int kTileE = 32;
+__device__ __forceinline__ void dft_tile(double2* cur, double2* nxt, const double2* wy, const double2* wz, int nky,
+                                         int nkz, bool inv) {
+  const int nk = nky * nkz;
+  for (int q = threadIdx.x; q < nk * kTileE; q += blockDim.x) {   // along kz
+    const int e = q % kTileE, k = q / kTileE, y = k / nkz, z = k % nkz;
+    double2 a = make_double2(0.0, 0.0);
+    for (int i = 0; i < nkz; i++) {
+      const double2 w = wz[(i * z) % nkz], v = cur[(y * nkz + i) * kTileE + e];
+      a = add(a, inv ? mulc(v, w) : mul(v, w));
+    }
+    nxt[q] = a;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < nk * kTileE; q += blockDim.x) {   // along ky
+    const int e = q % kTileE, k = q / kTileE, y = k / nkz, z = k % nkz;
+    double2 a = make_double2(0.0, 0.0);
+    for (int i = 0; i < nky; i++) {
+      const double2 w = wy[(i * y) % nky], v = nxt[(i * nkz + z) * kTileE + e];
+      a = add(a, inv ? mulc(v, w) : mul(v, w));
+    }
+    cur[q] = a;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(256) k_forward_any(Six in, const int64_t* __restrict__ lines, int64_t nl, Dims d,
+                                                     unsigned conj, const double2* __restrict__ ph,
+                                                     double2* __restrict__ kb) {
+  extern __shared__ __align__(16) double2 sh[];
+  const int nk = (int)d.nk, op = blockIdx.z;
+  const int64_t e0 = (int64_t)blockIdx.x * kTileE, b = blockIdx.y;
+  const double2* src = in.a[op] + lines[b] * nk * d.nen;
+  double2* dst = kb + ((size_t)op * nl + b) * nk * d.nen;
+  const double sg = (conj >> op) & 1 ? -1.0 : 1.0;
+  for (int q = threadIdx.x; q < nk * kTileE; q += blockDim.x) {
+    const int64_t e = e0 + q % kTileE;
+    const double2 v = e < d.nen ? src[(q / kTileE) * d.nen + e] : make_double2(0.0, 0.0);
+    sh[q] = make_double2(v.x, sg * v.y);
+  }
+  __syncthreads();
+  dft_tile(sh, sh + nk * kTileE, ph + nk, ph + nk + d.nky, (int)d.nky, (int)d.nkz, false);
+  for (int q = threadIdx.x; q < nk * kTileE; q += blockDim.x) {
+    const int64_t e = e0 + q % kTileE;
+    if (e < d.nen) dst[(q / kTileE) * d.nen + e] = sh[q];
+  }
+}
+
+__global__ void __launch_bounds__(256) k_inverse_any(Three out, const int64_t* __restrict__ lines, int64_t nl, Dims d,
+                                                     bool fix, const double2* __restrict__ ph,
+                                                     const double2* __restrict__ pb) {
+  extern __shared__ __align__(16) double2 sh[];
+  const int nk = (int)d.nk;
+  double* diff = (double*)(sh + 2 * nk * kTileE);
+  const int64_t e0 = (int64_t)blockIdx.x * kTileE, b = blockIdx.y;
+  for (int v = 0; v < 3; v++) {
+    const double2* src = pb + ((size_t)v * nl + b) * nk * d.nen;
+    double2* dst = out.a[v] + lines[b] * nk * d.nen;
+    for (int q = threadIdx.x; q < nk * kTileE; q += blockDim.x) {
+      const int64_t e = e0 + q % kTileE;
+      sh[q] = e < d.nen ? mul(src[(q / kTileE) * d.nen + e], ph[q / kTileE]) : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    dft_tile(sh, sh + nk * kTileE, ph + nk, ph + nk + d.nky, (int)d.nky, (int)d.nkz, true);
+    for (int q = threadIdx.x; q < nk * kTileE; q += blockDim.x) {
+      const int64_t e = e0 + q % kTileE;
+      double2 x = sh[q];
+      if (v == 0) diff[q] = -x.y;
+      else if (v == 1) diff[q] += x.y;
+      else if (fix) x.y = diff[q] / 2.0;
+      if (e < d.nen) dst[(q / kTileE) * d.nen + e] = x;
+    }
+    __syncthreads();
+  }
+}
+
+// Energy transforms, products and windows of (line, k-frequency) tasks.
+// The circular length is N = 2 M with M = 2^LOGM >= nen, and a task does its
+// even and its odd frequencies one after the other, each a problem of length
+// M: X[2f] is the M-point transform of x[n] + x[n + M], X[2f + 1] that of
+// (x[n] - x[n + M]) exp(-2 pi i n / N), and the result is E[n] +- exp(2 pi i
+// n / N) O[n] (n < M, n + M), of which the window needs one sign per n.  The
+// padding is then never transformed, M = 4096 takes two exchanges instead of
+// the three of 8192, and two CTAs fit an SM, so one exchanges while the other
+// computes.  Measured (1 B200, nen = 4096, 4 x 4 k-grid, 140 lines, P and
+// Sigma): cuFFT's 3-D form 9.8 ms; own transforms of N = 8192, one CTA an SM
+// 5.1 ms (these kernels 3.2 of it, the zeros outside the band 1.2); halves of
+// M = 4096 with the zeros written beside them 4.5 ms.
+//
+// NT = M / 16 threads a task, G tasks side by side in a CTA of at least 128
+// threads.  kb: operands [op][line][k][energy]; pb: windows [v][line][k]
+// [energy]; scr: three half spectra for each task in work (L2).  The
+// conjugate of the correlation's second operands was transformed, so their
+// spectra at negated frequencies are conjugates at the same ones:
+//   P^< = G^< conj(Y^>),  P^> = G^> conj(Y^<),
+//   P^R = G^< conj(G^R) + G^R conj(Y^<)      (the second operand conj(G^R))
+// and Sigma^R = G^< W^R + G^R (W^< + W^R).  Operands: P: G^<, G^>, G^R, Y^>,
+// Y^<; Sigma: G^<, G^>, G^R, W^<, W^>, W^R.
+// w: the twiddle table, w2: exp(-2 pi i n / N), n < M.
+template <int LOGM>
+struct Line {
+  using C = rgf::fft::Cfg<LOGM>;
+  static constexpr int kThreads = C::NT < 128 ? 128 : C::NT;
+  static constexpr int G = kThreads / C::NT;
+  static constexpr int kPerSm = 512 / kThreads;         // 128 registers a thread
+  static constexpr size_t smem = sizeof(double2) * G * C::SMEM;
+};
+
+template <int LOGM, int MODE>
+__global__ void __launch_bounds__(Line<LOGM>::kThreads, Line<LOGM>::kPerSm)
+line_kernel(int64_t nl, Dims d, const double2* __restrict__ w, const double2* __restrict__ w2,
+            const double2* __restrict__ kb, double2* __restrict__ pb, double2* __restrict__ scr) {
+  using C = rgf::fft::Cfg<LOGM>;
+  constexpr int M = C::M, NT = C::NT, G = Line<LOGM>::G;
+  extern __shared__ __align__(16) double2 sh[];
+  const int grp = threadIdx.x / NT, t = threadIdx.x % NT;
+  double2* buf = sh + grp * C::SMEM;
+  double2* s1 = scr + ((size_t)blockIdx.x * G + grp) * 3 * M + t;
+  double2 *s2 = s1 + M, *s3 = s2 + M;
+  const int nen = (int)d.nen, h = nen / 2;
+  const int64_t total = nl * d.nk, op_stride = total * nen;
+  const double2 zero = make_double2(0.0, 0.0);
+  double2 x[16];
+  for (int64_t base = (int64_t)blockIdx.x * G; base < total; base += (int64_t)gridDim.x * G) {
+    const int64_t task = base + grp;
+    const bool on = task < total;
+    const double2* in = kb + task * nen;
+    double2* out = pb + task * nen;
+#pragma unroll 1
+    for (int half = 0; half < 2; half++) {
+      auto load = [&](int op, bool shifted) {
+        const double2* src = in + op * op_stride;
+#pragma unroll
+        for (int m = 0; m < 16; m++) {
+          const int i = t + NT * m;
+          double2 v = zero;
+          if (!shifted) {              // a series, zero-padded
+            if (on && i < nen) v = __ldcg(src + i);
+          } else if (i < h) {          // W by its energy shift: n >= 0 first,
+            if (on) v = __ldcg(src + i + h - 1);
+          } else if (i > M - h) {      // n < 0 at the end of N (x[n + M])
+            if (on) v = __ldcg(src + i - M + h - 1);
+            if (half) v = make_double2(-v.x, -v.y);
+          }
+          x[m] = v;
+        }
+        if (half)
+#pragma unroll
+          for (int m = 0; m < 16; m++) x[m] = mul(x[m], w2[t + NT * m]);
+      };
+      auto keep = [&](double2* s) {
+#pragma unroll
+        for (int m = 0; m < 16; m++) __stcg(s + NT * m, x[m]);
+      };
+      // one transform of each direction in the code: a loop over the operands
+#pragma unroll 1
+      for (int step = 0; step < (MODE == 0 ? 5 : 6); step++) {
+        int v = -1;                    // output of this step
+        if constexpr (MODE == 0) {
+          load(step == 0 ? 4 : (step == 1 ? 1 : (step == 2 ? 2 : (step == 3 ? 0 : 3))), false);
+          rgf::fft::transform<LOGM, false>(x, buf, w, t);
+          if (step == 0) {
+            keep(s1);                  // Y^<
+          } else if (step == 1) {
+#pragma unroll
+            for (int m = 0; m < 16; m++) x[m] = mulc(x[m], __ldcg(s1 + NT * m));
+            v = 1;
+          } else if (step == 2) {
+            keep(s2);                  // G^R
+          } else if (step == 3) {
+            keep(s3);                  // G^<
+#pragma unroll
+            for (int m = 0; m < 16; m++) {
+              const double2 gr = __ldcg(s2 + NT * m);
+              x[m] = add(mulc(x[m], gr), mulc(gr, __ldcg(s1 + NT * m)));
+            }
+            v = 2;
+          } else {
+#pragma unroll
+            for (int m = 0; m < 16; m++) x[m] = mulc(__ldcg(s3 + NT * m), x[m]);
+            v = 0;
+          }
+        } else {
+          load(step == 0 ? 4 : (step == 1 ? 1 : (step == 2 ? 3 : (step == 3 ? 5 : (step == 4 ? 0 : 2)))),
+               step == 0 || step == 2 || step == 3);
+          rgf::fft::transform<LOGM, false>(x, buf, w, t);
+          if (step == 0 || step == 2) {
+            keep(s1);                  // W^>, then W^<
+          } else if (step == 1) {
+#pragma unroll
+            for (int m = 0; m < 16; m++) x[m] = mul(x[m], __ldcg(s1 + NT * m));
+            v = 1;
+          } else if (step == 3) {
+            keep(s2);                  // W^R
+          } else if (step == 4) {
+            keep(s3);                  // G^<
+#pragma unroll
+            for (int m = 0; m < 16; m++) x[m] = mul(x[m], __ldcg(s1 + NT * m));
+            v = 0;
+          } else {
+#pragma unroll
+            for (int m = 0; m < 16; m++) {
+              const double2 wr = __ldcg(s2 + NT * m);
+              x[m] = add(mul(__ldcg(s3 + NT * m), wr), mul(x[m], add(__ldcg(s1 + NT * m), wr)));
+            }
+            v = 2;
+          }
+        }
+        if (v < 0) continue;
+        rgf::fft::transform<LOGM, true>(x, buf, w, t);
+        if (!on) continue;
+        double2* dst = out + v * op_stride;
+#pragma unroll
+        for (int m = 0; m < 16; m++) {
+          const int i = t + NT * m;
+          // P(o): energy shift o - h, negative ones at n + M (minus sign)
+          const bool up = MODE == 0 && i >= M - h;
+          const int o = MODE == 1 ? i : (up ? i - (M - h) : (i < h ? i + h : nen));
+          if (o >= nen) continue;
+          if (half == 0) {
+            __stcg(dst + o, x[m]);
+          } else {
+            const double2 e = __ldcg(dst + o), q = mulc(x[m], w2[i]);
+            __stcg(dst + o, up ? rgf::fft::sub(e, q) : add(e, q));
+          }
+        }
+      }
+    }
+  }
+}
+
+}  // namespace own
+
 struct Plan {
   cufftHandle h = 0;
   bool created = false, ok = false;
@@ -177,6 +516,17 @@ struct FftCache {
   std::unique_ptr<struct Plan> full, part;
   void* scratch = nullptr;
   size_t bytes = 0;
+  double2* roots[own::kMaxLog + 1] = {};   // own transforms: exp(-2 pi i n / 2M), n < M, then the twiddles
+  int roots_dev = -1;
+  cudaStream_t fill = nullptr;             // zeroes the elements outside the band beside the transforms
+  cudaEvent_t fill_from = nullptr;
+  int fill_dev = -1;
+  void close_fill() {
+    if (fill) cudaStreamDestroy(fill);
+    if (fill_from) cudaEventDestroy(fill_from);
+    fill = nullptr;
+    fill_from = nullptr;
+  }
   ~FftCache();
   static void destroy(void* p) { delete static_cast<FftCache*>(p); }
 };
@@ -184,6 +534,9 @@ struct FftCache {
 FftCache::~FftCache() {
   full.reset();
   part.reset();
+  for (double2* r : roots)
+    if (r) cudaFree(r);
+  close_fill();
   if (scratch) {
     int cur = 0;
     cudaGetDevice(&cur);
@@ -191,6 +544,176 @@ FftCache::~FftCache() {
     cudaFree(scratch);
     cudaSetDevice(cur);
   }
+}
+
+// cache->scratch of at least `need` bytes on device dev
+int reserve_scratch(FftCache* cache, int dev, size_t need, cudaStream_t st) {
+  if (cache->dev == dev && cache->bytes >= need) return RGF_OK;
+  cudaError_t e = cudaStreamSynchronize(st);   // earlier calls may still use the old scratch
+  if (cache->scratch) cudaFree(cache->scratch);
+  cache->scratch = nullptr;
+  cache->bytes = 0;
+  if (e == cudaSuccess) e = cudaMalloc(&cache->scratch, need);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    cache->scratch = nullptr;
+    return fft_fail(RGF_E_NOMEM, "device scratch for the transforms");
+  }
+  cache->bytes = need;
+  return RGF_OK;
+}
+
+// exp(-2 pi i num / den), rounded once
+double2 unit_root(int64_t num, int64_t den) {
+  const long double th = 2.0L * 3.14159265358979323846264338327950288L * (long double)num / (long double)den;
+  return make_double2((double)cosl(th), (double)-sinl(th));
+}
+
+// ---- the library's own transforms
+using LineFn = void (*)(int64_t, Dims, const double2*, const double2*, const double2*, double2*, double2*);
+struct LineLaunch {
+  LineFn fn[2];
+  int threads, group, per_sm;
+  size_t smem;
+};
+template <int LOGM>
+LineLaunch line_launch() {
+  using L = own::Line<LOGM>;
+  return LineLaunch{{own::line_kernel<LOGM, 0>, own::line_kernel<LOGM, 1>}, L::kThreads, L::G, L::kPerSm, L::smem};
+}
+LineLaunch line_launch_for(int logm) {
+  switch (logm) {
+    case 5: return line_launch<5>();
+    case 6: return line_launch<6>();
+    case 7: return line_launch<7>();
+    case 8: return line_launch<8>();
+    case 9: return line_launch<9>();
+    case 10: return line_launch<10>();
+    case 11: return line_launch<11>();
+    default: return line_launch<12>();
+  }
+}
+
+constexpr int64_t kAnyGridMaxK = 160;   // tile of the general k-grid kernels: 40 KB a k-point x 32 energies
+// log2 M, or 0 where the form does not apply
+int own_log(const Dims& d) {
+  if (d.nk > kAnyGridMaxK) return 0;
+  for (int l = own::kMinLog; l <= own::kMaxLog; l++)
+    if ((int64_t(1) << l) >= d.nen) return l;
+  return 0;
+}
+
+template <int NKY, int NKZ>
+void launch_k(bool forward, const own::Six& in, const own::Three& out, const int64_t* lines, int64_t nl, const Dims& d,
+              int nops, unsigned conj, bool fix, const double2* ph, double2* kb, const double2* pb, cudaStream_t st) {
+  if (forward)
+    own::k_forward<NKY, NKZ><<<dim3((unsigned)((d.nen + 255) / 256), (unsigned)nl, (unsigned)nops), 256, 0, st>>>(
+        in, lines, nl, d, conj, kb);
+  else
+    own::k_inverse<NKY, NKZ><<<dim3((unsigned)((d.nen + 127) / 128), (unsigned)nl), 128, 0, st>>>(out, lines, nl, d,
+                                                                                                fix, ph, pb);
+}
+
+void k_transform(bool forward, const own::Six& in, const own::Three& out, const int64_t* lines, int64_t nl,
+                 const Dims& d, int nops, unsigned conj, bool fix, const double2* ph, double2* kb, const double2* pb,
+                 cudaStream_t st) {
+#define RGF_K_CASE(Y, Z) \
+  if (d.nky == Y && d.nkz == Z) return launch_k<Y, Z>(forward, in, out, lines, nl, d, nops, conj, fix, ph, kb, pb, st)
+  RGF_K_CASE(1, 1);
+  RGF_K_CASE(1, 2);
+  RGF_K_CASE(2, 1);
+  RGF_K_CASE(2, 2);
+  RGF_K_CASE(1, 4);
+  RGF_K_CASE(4, 1);
+  RGF_K_CASE(2, 4);
+  RGF_K_CASE(4, 2);
+  RGF_K_CASE(4, 4);
+#undef RGF_K_CASE
+  const size_t tile = (size_t)d.nk * own::kTileE * sizeof(double2);
+  const unsigned ge = (unsigned)((d.nen + own::kTileE - 1) / own::kTileE);
+  if (forward) {
+    cudaFuncSetAttribute(own::k_forward_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * tile));
+    own::k_forward_any<<<dim3(ge, (unsigned)nl, (unsigned)nops), 256, 2 * tile, st>>>(in, lines, nl, d, conj, ph, kb);
+  } else {
+    cudaFuncSetAttribute(own::k_inverse_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * tile + tile / 2));
+    own::k_inverse_any<<<dim3(ge, (unsigned)nl), 256, 2 * tile + tile / 2, st>>>(out, lines, nl, d, fix, ph, pb);
+  }
+}
+
+// ph: the nk phases, then the nky-th and nkz-th roots.
+int run_own(FftCache* cache, int dev, int mode, const Dims& d, int logm, const std::vector<int64_t>& lines,
+            const std::vector<double2>& ph, const double2* const in[6], double2* const out[3], cudaStream_t st) {
+  const int64_t M = int64_t(1) << logm;
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const LineLaunch L = line_launch_for(logm);
+  const int nops = mode == 0 ? 5 : 6;
+  const size_t per_line = (size_t)(nops + 3) * d.nk * d.nen;   // values
+  const int64_t nl = (int64_t)lines.size();
+  int64_t chunk = (int64_t)(((size_t)1 << 30) / sizeof(double2) / per_line);
+  if (const char* env = std::getenv("RGF_GW_FFT_CHUNK")) {
+    const long v = std::atol(env);
+    if (v > 0) chunk = v;
+  }
+  chunk = chunk < 1 ? 1 : (chunk > nl ? nl : chunk);
+  if (chunk > 65535) chunk = 65535;                             // grid y
+  const int64_t ctas = (int64_t)sms * L.per_sm;
+  const size_t scr = (size_t)ctas * L.group * 3 * M;
+  int rc = reserve_scratch(cache, dev, sizeof(double2) * (per_line * chunk + scr + ph.size()) + sizeof(int64_t) * nl, st);
+  if (rc) return rc;
+  cache->dev = dev;
+  if (cache->roots_dev != dev) {
+    for (double2*& r : cache->roots) {
+      if (r) cudaFree(r);
+      r = nullptr;
+    }
+    cache->roots_dev = dev;
+  }
+  if (!cache->roots[logm]) {
+    std::vector<double2> r((size_t)M);
+    for (int64_t n = 0; n < M; n++) r[n] = unit_root(n, 2 * M);
+    r.resize((size_t)M + rgf::fft::table(logm, [](int, long long, long long) {}));
+    rgf::fft::table(logm, [&](int k, long long num, long long den) { r[M + k] = unit_root(num, den); });
+    double2* p = nullptr;
+    if (cudaMalloc(&p, sizeof(double2) * r.size()) != cudaSuccess) {
+      cudaGetLastError();
+      return fft_fail(RGF_E_NOMEM, "table of roots");
+    }
+    if (cudaMemcpy(p, r.data(), sizeof(double2) * r.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaFree(p);
+      return fft_fail(RGF_E_CUDA, "table of roots");
+    }
+    cache->roots[logm] = p;
+  }
+  double2* kb = (double2*)cache->scratch;
+  double2* pb = kb + (size_t)nops * chunk * d.nk * d.nen;
+  double2* d_scr = pb + (size_t)3 * chunk * d.nk * d.nen;
+  double2* d_ph = d_scr + scr;
+  int64_t* d_lines = (int64_t*)(d_ph + ph.size());
+  cudaError_t ce = cudaMemcpyAsync(d_lines, lines.data(), sizeof(int64_t) * nl, cudaMemcpyHostToDevice, st);
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_ph, ph.data(), sizeof(double2) * ph.size(), cudaMemcpyHostToDevice, st);
+  // the host vectors must outlive the asynchronous copies from them
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+  if (ce == cudaSuccess && L.smem > 48 * 1024)
+    ce = cudaFuncSetAttribute(L.fn[mode], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
+  if (ce != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(ce));
+  own::Six src;
+  for (int a = 0; a < 6; a++) src.a[a] = in[a];
+  const own::Three dst{{out[0], out[1], out[2]}};
+  const unsigned conj = mode == 0 ? 0x18u : 0u;                 // Y^>, Y^<
+  for (int64_t c0 = 0; c0 < nl; c0 += chunk) {
+    const int64_t nb = (nl - c0) < chunk ? (nl - c0) : chunk;
+    const int64_t tasks = nb * d.nk, need = (tasks + L.group - 1) / L.group;
+    k_transform(true, src, dst, d_lines + c0, nb, d, nops, conj, false, d_ph, kb, pb, st);
+    L.fn[mode]<<<(unsigned)(need < ctas ? need : ctas), L.threads, L.smem, st>>>(
+        nb, d, cache->roots[logm] + M, cache->roots[logm], kb, pb, d_scr);
+    k_transform(false, src, dst, d_lines + c0, nb, d, nops, conj, mode == 1, d_ph, kb, pb, st);
+    ce = cudaGetLastError();
+    if (ce != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(ce));
+  }
+  ce = cudaStreamSynchronize(st);
+  if (ce != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(ce));
+  return RGF_OK;
 }
 
 unsigned grid_for(int64_t total) {
@@ -220,12 +743,6 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
   if (d.N > (1 << 30) || d.nky > (1 << 20) || d.nkz > (1 << 20))
     return fft_fail(RGF_E_UNSUPPORTED, "transform length out of range");
   const size_t series = (size_t)d.nk * nen;
-  // zero every output (elements outside the band stay zero, as the
-  // reference's zeroed buffers do)
-  for (int a = 0; a < 3; a++) {
-    const cudaError_t e = cudaMemsetAsync(out[a], 0, sizeof(double2) * series * nx * nij, st);
-    if (e != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(e));
-  }
   // banded lines (i, ix), line = i * nx + ix (src/green_rgf.f90:1401-1408)
   std::vector<int64_t> lines;
   for (int64_t i = 0; i < nij; i++) {
@@ -235,12 +752,58 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
     if (col < lo || col > hi) continue;
     for (int64_t ix = 0; ix < nx; ix++) lines.push_back(i * nx + ix);
   }
+  // elements outside the band are zero, as in the reference's zeroed buffers:
+  // the runs of elements between banded ones, or everything where the runs
+  // are many
+  std::vector<std::pair<int64_t, int64_t>> gaps;
+  for (size_t q = 0; q <= lines.size(); q += nx) {
+    const int64_t from = q == 0 ? 0 : lines[q - nx] / nx + 1, to = q < lines.size() ? lines[q] / nx : nij;
+    if (to > from) gaps.push_back({from, to});
+  }
+  if (gaps.size() > 64) gaps.assign(1, {0, nij});
+  int dev = 0;
+  cudaGetDevice(&dev);
+  FftCache* cache = static_cast<FftCache*>(rgf::ctx_ext_cache(ctx));
+  if (!cache) {
+    cache = new FftCache();
+    rgf::ctx_set_ext_cache(ctx, cache, &FftCache::destroy);
+  }
+  // the zeros are bound by HBM writes, the transforms by the SMs: they run
+  // beside each other, ordered after the caller's earlier work and complete
+  // before the call returns, whichever way it does
+  if (cache->fill_dev != dev) {
+    cache->close_fill();
+    if (cudaStreamCreateWithFlags(&cache->fill, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&cache->fill_from, cudaEventDisableTiming) != cudaSuccess) {
+      cache->close_fill();
+      return fft_fail(RGF_E_CUDA, "fill stream");
+    }
+    cache->fill_dev = dev;
+  }
+  struct FillDone {
+    cudaStream_t s;
+    ~FillDone() { cudaStreamSynchronize(s); }
+  } fill_done{cache->fill};
+  cudaError_t fe = cudaEventRecord(cache->fill_from, st);
+  if (fe == cudaSuccess) fe = cudaStreamWaitEvent(cache->fill, cache->fill_from, 0);
+  for (int a = 0; a < 3 && fe == cudaSuccess; a++)
+    for (const auto& r : gaps) {
+      fe = cudaMemsetAsync(out[a] + series * nx * r.first, 0, sizeof(double2) * series * nx * (r.second - r.first),
+                           cache->fill);
+      if (fe != cudaSuccess) break;
+    }
+  // a single run over everything includes the lines: they are written after it
+  if (fe == cudaSuccess && gaps.size() == 1 && gaps[0].first == 0 && gaps[0].second == nij)
+    fe = cudaStreamSynchronize(cache->fill);
+  if (fe != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(fe));
   if (lines.empty()) return RGF_OK;
   // the k-shift phase with the normalisation and dE folded in
   const double kPi = 3.14159265359;   // the reference's pi (src/green_rgf.f90:23)
   double2 dE;
   if (mode == 0) dE = make_double2(0.0, -1.0 * dEn / 2.0 / kPi * spindeg / (double)d.nk);
   else dE = make_double2(0.0, dEn / 2.0 / kPi / (double)d.nk);
+  const int logm = own_log(d);
+  if (logm) d.N = int64_t(2) << logm;
   const double norm = 1.0 / ((double)d.nk * (double)d.N);
   const double sgn = mode == 0 ? -1.0 : 1.0;
   const int64_t sy = nky > 1 ? ((nky / 2 - 1) % nky + nky) % nky : 0;
@@ -251,6 +814,11 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
     const double th = sgn * 2.0 * M_PI * ((double)(ky * sy) / (double)nky + (double)(kz * sz) / (double)nkz);
     const double2 e = make_double2(std::cos(th) * norm, std::sin(th) * norm);
     ph[k] = make_double2(e.x * dE.x - e.y * dE.y, e.x * dE.y + e.y * dE.x);
+  }
+  if (logm) {
+    for (int64_t n : {nky, nkz})
+      for (int64_t m = 0; m < n; m++) ph.push_back(unit_root(m, n));
+    return run_own(cache, dev, mode, d, logm, lines, ph, in, out, st);
   }
   // chunk of lines: six spectra of nk x N complex values each
   const size_t per_line = 6 * (size_t)d.nk * d.N * sizeof(double2);
@@ -265,26 +833,9 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
   if (chunk > cap) chunk = cap;
   if (chunk < 1) return fft_fail(RGF_E_UNSUPPORTED, "one line exceeds the transform size limit");
   const int64_t nl = (int64_t)lines.size();
-  int dev = 0;
-  cudaGetDevice(&dev);
-  FftCache* cache = static_cast<FftCache*>(rgf::ctx_ext_cache(ctx));
-  if (!cache) {
-    cache = new FftCache();
-    rgf::ctx_set_ext_cache(ctx, cache, &FftCache::destroy);
-  }
   const size_t need = per_line * chunk + sizeof(int64_t) * lines.size() + sizeof(double2) * d.nk;
-  if (cache->dev != dev || cache->bytes < need) {
-    cudaError_t e = cudaStreamSynchronize(st);   // earlier calls may still use the old scratch
-    if (cache->scratch) cudaFree(cache->scratch);
-    cache->scratch = nullptr;
-    cache->bytes = 0;
-    if (e == cudaSuccess) e = cudaMalloc(&cache->scratch, need);
-    if (e != cudaSuccess) {
-      cache->scratch = nullptr;
-      return fft_fail(RGF_E_NOMEM, "device scratch for the transforms");
-    }
-    cache->bytes = need;
-  }
+  const int rc = reserve_scratch(cache, dev, need, st);
+  if (rc) return rc;
   const int64_t tail = nl % chunk;
   if (cache->dev != dev || cache->nky != nky || cache->nkz != nkz || cache->N != d.N || cache->chunk != chunk ||
       cache->tail != tail || !cache->full) {
@@ -308,8 +859,10 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
   const size_t spec = (size_t)chunk * d.nk * d.N;
   double2* buf[6];
   for (int a = 0; a < 6; a++) buf[a] = (double2*)cache->scratch + a * spec;
-  int64_t* d_lines = (int64_t*)((double2*)cache->scratch + 6 * spec);
-  double2* d_ph = (double2*)(d_lines + lines.size());
+  // the phases before the line numbers: an odd count of those would leave
+  // 16-byte values at an odd multiple of 8
+  double2* d_ph = (double2*)cache->scratch + 6 * spec;
+  int64_t* d_lines = (int64_t*)(d_ph + d.nk);
   cudaError_t ce = cudaMemcpyAsync(d_lines, lines.data(), sizeof(int64_t) * lines.size(), cudaMemcpyHostToDevice, st);
   if (ce == cudaSuccess) ce = cudaMemcpyAsync(d_ph, ph.data(), sizeof(double2) * d.nk, cudaMemcpyHostToDevice, st);
   if (ce != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(ce));
