@@ -220,8 +220,9 @@ RGF_API int rgf_plan_destroy(rgf_plan* plan);
 
 /* Autotuner.  No counterpart in the reference.  For the block size of
  * `device`, times every kernel variant that supports it (staged GEMM with
- * blocked inverse for nb = 32, 64, 128, 256; register-direct GEMMs with 8x8,
- * 8x16 and 16x16 warp tiles for any multiple of 8 / 16) at 1 and at the
+ * blocked inverse for nb = 32, 64, 128, 256; the same with run-time tiles for
+ * the other multiples of 8 from 80 on; register-direct GEMMs with 8x8, 8x16
+ * and 16x16 warp tiles for any multiple of 8 / 16) at 1 and at the
  * largest number of resident CTAs per SM, each on a probe batch of the
  * device's first min(nx, 12) blocks with one energy per resident CTA
  * (outputs G^R_ll, G^<_ll, T; energies spread over [-3, 3] eV), and keeps the

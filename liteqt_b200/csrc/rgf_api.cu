@@ -1050,6 +1050,15 @@ static int launch_ctas_per_sm(const rgf_ctx* c, size_t smem, uint64_t nb_mask) {
   return k;
 }
 
+// Geometry of a launch over n_tasks tasks of the block sizes in nb_mask: as
+// many CTAs as are resident at a time, one a task.
+static SolverShape solver_shape(const rgf_ctx* c, size_t smem, uint64_t nb_mask, int64_t n_tasks) {
+  SolverShape s;
+  s.groups = (int)std::min<int64_t>(c->sm_count * launch_ctas_per_sm(c, smem, nb_mask), n_tasks);
+  s.smem = smem;
+  return s;
+}
+
 // Checks a task list; RGF_OK or the error.
 static int validate_batch(const rgf_device* devices, int32_t n_devices, const rgf_task* tasks,
                           int64_t n_tasks) {
@@ -1239,8 +1248,8 @@ extern "C" int rgf_solve_batch(rgf_ctx* c, const rgf_device* devices, int32_t n_
   const LaunchShape shape = launch_shape(c, devices, tasks, n_tasks);
   const std::vector<int32_t>& order = shape.order;
   int64_t slot = shape.slot;
-  const size_t smem = shape.smem;
-  int grid = c->sm_count * launch_ctas_per_sm(c, smem, shape.nb_mask);
+  const SolverShape geo = solver_shape(c, shape.smem, shape.nb_mask, n_tasks);
+  int grid = geo.groups;
   if (mixed) {
     int64_t nx_max = 2;
     for (int32_t d = 0; d < n_devices; d++) nx_max = std::max<int64_t>(nx_max, devices[d].nx);
@@ -1293,7 +1302,7 @@ extern "C" int rgf_solve_batch(rgf_ctx* c, const rgf_device* devices, int32_t n_
     RGF_CUDA(cudaHostGetDevicePointer((void**)&p.progress, c->sync_prog, 0));
   }
   RGF_CUDA(cudaEventRecord(c->ev0, st));
-  cudaError_t e = mixed ? launch_mixed(p, grid, st) : launch_solver(p, grid, smem, st);
+  cudaError_t e = mixed ? launch_mixed(p, grid, st) : launch_solver(p, geo, st);
   if (e != cudaSuccess) return fail(RGF_E_CUDA, "solver launch failed: %s", cudaGetErrorString(e));
   c->stats.launches++;
   RGF_CUDA(cudaEventRecord(c->ev1, st));
@@ -1496,10 +1505,9 @@ extern "C" int rgf_adjoint_energies(rgf_ctx* c, const rgf_device* v, int64_t nen
   RGF_CUDA(cudaMemsetAsync(c->info.p, 0, sizeof(DInfo) * nen, st));
   RGF_CUDA(cudaMemsetAsync(c->queue.p, 0, sizeof(int32_t), st));
   const size_t smem = variant_smem(c->variant[nm / 8], (int)nm);
-  int grid = c->sm_count * launch_ctas_per_sm(c, smem, 1ull << (nm / 8));
-  if ((int64_t)grid > nen) grid = (int)nen;
+  const SolverShape geo = solver_shape(c, smem, 1ull << (nm / 8), nen);
   const int64_t slot = slot_elems_for(nm, nx);
-  if ((rc = c->work.reserve(sizeof(double2) * (size_t)slot * grid))) return rc;
+  if ((rc = c->work.reserve(sizeof(double2) * (size_t)slot * geo.groups))) return rc;
   KParams p;
   fill_params(c, p);
   p.o.want_T = 1;
@@ -1511,7 +1519,7 @@ extern "C" int rgf_adjoint_energies(rgf_ctx* c, const rgf_device* v, int64_t nen
   p.info = (DInfo*)c->info.p;
   p.adj = (const DAdj*)tb;
   RGF_CUDA(cudaEventRecord(c->ev0, st));
-  cudaError_t e = launch_solver(p, grid, smem, st);
+  cudaError_t e = launch_solver(p, geo, st);
   if (e != cudaSuccess) return fail(RGF_E_CUDA, "adjoint launch failed: %s", cudaGetErrorString(e));
   c->stats.launches++;
   RGF_CUDA(cudaEventRecord(c->ev1, st));
@@ -1943,9 +1951,8 @@ extern "C" int rgf_plan_create(rgf_ctx* c, const rgf_device* devices, int32_t n_
     pl->task_nb[t] = (int)devices[k.device].nm;
   }
   const LaunchShape shape = launch_shape(c, devices, tasks, n_tasks);
-  int grid = c->sm_count * launch_ctas_per_sm(c, shape.smem, shape.nb_mask);
-  if ((int64_t)grid > n_tasks) grid = (int)n_tasks;
-  if ((rc = pl->work.reserve(sizeof(double2) * (size_t)shape.slot * grid))) return rc;
+  const SolverShape geo = solver_shape(c, shape.smem, shape.nb_mask, n_tasks);
+  if ((rc = pl->work.reserve(sizeof(double2) * (size_t)shape.slot * geo.groups))) return rc;
   if ((rc = pl->devs.reserve(sizeof(DDev) * n_devices))) return rc;
   if ((rc = pl->tasks.reserve(sizeof(DTask) * n_tasks + sizeof(int32_t) * n_tasks))) return rc;
   if ((rc = pl->info.reserve(sizeof(DInfo) * n_tasks))) return rc;
@@ -1964,14 +1971,14 @@ extern "C" int rgf_plan_create(rgf_ctx* c, const rgf_device* devices, int32_t n_
   p.work = (double2*)pl->work.p;
   p.slot_elems = shape.slot;
   p.info = (DInfo*)pl->info.p;
-  solver_blocks_per_sm(shape.smem);  // raises the kernel's shared-memory limit before the capture
+  solver_blocks_per_sm(geo.smem);  // raises the kernel's shared-memory limit before the capture
   cudaStream_t cs = nullptr;
   RGF_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
     cudaError_t e1 = cudaMemsetAsync(pl->queue.p, 0, sizeof(int32_t), cs);
     cudaError_t e2 = cudaMemsetAsync(pl->info.p, 0, sizeof(DInfo) * n_tasks, cs);
-    cudaError_t e3 = launch_solver(p, grid, shape.smem, cs, false);
+    cudaError_t e3 = launch_solver(p, geo, cs, false);
     e = cudaStreamEndCapture(cs, &pl->graph);
     if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
   }
@@ -2201,9 +2208,8 @@ extern "C" int rgf_w_solve_batch(rgf_ctx* c, const rgf_w_device* devices, int32_
     nb_mask |= 1ull << (v.nm / 8);
   }
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
-  int grid = c->sm_count * launch_ctas_per_sm(c, smem, nb_mask);
-  if ((int64_t)grid > n_tasks) grid = (int)n_tasks;
-  if ((rc = c->work.reserve(sizeof(double2) * (size_t)slot * grid))) return rc;
+  const SolverShape geo = solver_shape(c, smem, nb_mask, n_tasks);
+  if ((rc = c->work.reserve(sizeof(double2) * (size_t)slot * geo.groups))) return rc;
   if ((rc = c->devs.reserve(sizeof(DDev) * n_devices))) return rc;
   if ((rc = c->tasks.reserve(sizeof(DWTask) * n_tasks + sizeof(int32_t) * n_tasks))) return rc;
   if ((rc = c->info.reserve(sizeof(DInfo) * n_tasks))) return rc;
@@ -2225,7 +2231,7 @@ extern "C" int rgf_w_solve_batch(rgf_ctx* c, const rgf_w_device* devices, int32_
   p.info = (DInfo*)c->info.p;
   p.wtasks = (const DWTask*)c->tasks.p;
   RGF_CUDA(cudaEventRecord(c->ev0, st));
-  cudaError_t e = launch_solver(p, grid, smem, st);
+  cudaError_t e = launch_solver(p, geo, st);
   if (e != cudaSuccess) return fail(RGF_E_CUDA, "W launch failed: %s", cudaGetErrorString(e));
   c->stats.launches++;
   RGF_CUDA(cudaEventRecord(c->ev1, st));

@@ -21,6 +21,27 @@ namespace rgf {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 
+// The CTAs that work on one task: a single one, or a cluster of them.
+struct Group {
+  int rank = 0, size = 1;
+  // Barrier over the group; what its threads wrote to global memory before is
+  // visible to all of them after it (cluster barriers order arrive.release
+  // before wait.acquire).  Every thread of every CTA of the group calls it.
+  __device__ __forceinline__ void sync() const {
+    if (size == 1) {
+      __syncthreads();
+    } else {
+      asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+  }
+};
+
+// A task of one CTA, known at compile time.
+struct SoloGroup {
+  static constexpr int rank = 0, size = 1;
+  __device__ __forceinline__ void sync() const { __syncthreads(); }
+};
+
 // ---------------------------------------------------------------- complex
 __device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
@@ -32,7 +53,11 @@ __device__ __forceinline__ double2 cscale(double2 a, double s) { return make_dou
 __device__ __forceinline__ double2 czero() { return make_double2(0.0, 0.0); }
 // 1/(a+ib) = (a-ib) / (a^2+b^2).  a and b are first scaled by the power of
 // two 2^-e (exact) that brings max(|a|, |b|) into [1/2, 1), so the squares
-// neither overflow nor underflow, and one division forms 1/(a^2+b^2).  Zero,
+// neither overflow nor underflow and d = a^2 + b^2 lies in [1/4, 2).  1/d is
+// one step of Halley's iteration from a single-precision reciprocal r: with
+// e = 1 - d r, |e| < 2^-21, r + r (e + e^2) is 1/d to e^3 < 2^-63 before its
+// own rounding -- a chain of three FP64 operations in the elimination's
+// critical path, where the division's is about three times as long.  Zero,
 // subnormal, infinite and NaN arguments and exponents near the ends of the
 // range take the quotient form with two divisions.
 __device__ __forceinline__ double2 crecip(double2 a) {
@@ -45,7 +70,11 @@ __device__ __forceinline__ double2 crecip(double2 a) {
   }
   const double sc = __longlong_as_double((long long)(1023 - e) << 52);  // 2^-e
   const double ar = a.x * sc, ai = a.y * sc;
-  const double r = 1.0 / (ar * ar + ai * ai);
+  const double d = ar * ar + ai * ai;
+  float f;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"((float)d));
+  const double r0 = (double)f, t = fma(-d, r0, 1.0);
+  const double r = fma(r0, fma(t, t, t), r0);
   return make_double2(ar * r * sc, -ai * r * sc);
 }
 // |re| + |im|: the pivot measure of LAPACK's izamax (dcabs1), used by zgetrf.

@@ -75,11 +75,14 @@ struct DAdj {
 
 // Block-operation policies ("kernel variants") a task can run with:
 // staged = shared-memory-staged GEMM + blocked inverse for one block size;
-// generic = register-direct GEMM with TM x TN warp tiles for any multiple of 8.
+// generic = register-direct GEMM with TM x TN warp tiles for any multiple of 8
+// (1x1) or 16; tiled = staged GEMM in tiles that follow a block size known at
+// run time, blocked inverse.
 enum KVariant : int {
   KV_NONE = -1,
   KV_STAGED32 = 0, KV_STAGED64, KV_STAGED128, KV_STAGED256,
   KV_GENERIC11, KV_GENERIC12, KV_GENERIC22,
+  KV_TILED,
   KV_COUNT
 };
 constexpr int kVariantSlots = kMaxNb / 8 + 1;  // indexed by nb / 8
@@ -105,7 +108,7 @@ struct KParams {
   int64_t n_tasks;
   const int32_t* order;    // task order of the queue (longest first), or NULL
   int32_t* queue;          // work-queue counter (zeroed before launch)
-  double2* work;           // workspace: one slot per resident CTA
+  double2* work;           // workspace: one slot per resident CTA (per cluster, where a cluster shares a task)
   int64_t slot_elems;      // complex elements per slot (>= slot_elems_for(nb, nx) of every task)
   DInfo* info;             // per task
   int32_t* progress;       // per task, or NULL: blocks whose outputs are written, counted from
@@ -131,11 +134,18 @@ void set_default_variants(KParams& p);
 // Max resident CTAs per SM of the solver kernel with this much dynamic
 // shared memory (occupancy query).
 int solver_blocks_per_sm(size_t smem);
+// Clusters of `cluster` CTAs of the solver kernel that fit the GPU at a time.
+int solver_max_clusters(size_t smem, int cluster);
+// Geometry of a solver launch: `groups` work slots, each drained by one CTA
+// or by a cluster of CTAs that share every task.
+struct SolverShape {
+  int groups = 1, cluster = 1;
+  size_t smem = 0;
+};
 // Launch the persistent solver over all tasks of p (any mix of block sizes).
 // set_attr = false skips raising the kernel's dynamic shared-memory limit
 // (inside a stream capture, after solver_blocks_per_sm(smem) has done it).
-cudaError_t launch_solver(const KParams& p, int grid, size_t smem, cudaStream_t stream,
-                          bool set_attr = true);
+cudaError_t launch_solver(const KParams& p, const SolverShape& s, cudaStream_t stream, bool set_attr = true);
 int solver_threads();
 
 // Mixed-precision form (rgf_mixed.cu): nb = 128, one CTA per SM.

@@ -302,7 +302,7 @@ struct MixState {
 // refined FP32 inverse while `mixed_on`, the plain FP64 operations
 // (StagedOps<128>) otherwise (Sancho-Rubio and its self-energies).
 struct MixedOps {
-  static constexpr bool kMixed = true;
+  static constexpr bool kMixed = true, kGroup = false;
   static constexpr int kMinBlocks = 1;
   StagedOps<128> f64;
   SmemInv& inv;

@@ -179,7 +179,10 @@ extern "C" int rgf_solve_energies_noalloc(const rgf_opts* opts, const rgf_device
   p.work = (double2*)(base + off_slots);
   p.slot_elems = slot_elems_for(nm, nx);
   p.info = (DInfo*)(base + off_info);
-  NA_CUDA(launch_solver(p, (int)grid, smem, st));
+  SolverShape shape;
+  shape.groups = (int)grid;
+  shape.smem = smem;
+  NA_CUDA(launch_solver(p, shape, st));
   std::vector<DInfo> hinfo((size_t)nen);
   NA_CUDA(cudaMemcpyAsync(hinfo.data(), base + off_info, sizeof(DInfo) * (size_t)nen, cudaMemcpyDeviceToHost, st));
   NA_CUDA(cudaStreamSynchronize(st));

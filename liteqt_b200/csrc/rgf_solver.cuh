@@ -40,6 +40,7 @@
 #include "rgf_internal.h"
 #include "rgf_staged.cuh"
 #include "rgf_tasks.h"
+#include "rgf_tiled.cuh"
 
 namespace rgf {
 
@@ -63,11 +64,11 @@ static_assert(T_COUNT <= kNumTemps, "temp blocks");
 
 constexpr int kSmemXMaxNb = 64;  // generic path: inverse workspace in shared memory up to this nb
 
-// Any nb that is a multiple of 8: register-direct DMMA GEMM (warp tiles of
-// TM x TN 8x8 subtiles), unblocked Gauss-Jordan.
+// Register-direct DMMA GEMM (warp tiles of TM x TN 8x8 subtiles), unblocked
+// Gauss-Jordan; one CTA a task.
 template <int TM, int TN>
 struct GenericOps {
-  static constexpr bool kMixed = false;
+  static constexpr bool kMixed = false, kGroup = false;
   static constexpr int kMinBlocks = 2;
   static size_t smem_bytes(int nb) {
     return ((nb <= kSmemXMaxNb ? (size_t)nb * nb : 0) + 2 * (size_t)nb) * sizeof(double2);
@@ -75,7 +76,7 @@ struct GenericOps {
   SmemInv& inv;
   double2* X;
   double2* rowk;
-  __device__ GenericOps(SmemInv& i, double2* dyn, double2* slot_inv, double2*, int n)
+  __device__ GenericOps(SmemInv& i, double2* dyn, double2* slot_inv, double2*, int n, Group = Group{})
       : inv(i), X(n <= kSmemXMaxNb ? dyn : slot_inv),
         rowk(dyn + (n <= kSmemXMaxNb ? (size_t)n * n : 0)) {}
   template <class Epi>
@@ -93,30 +94,67 @@ struct GenericOps {
 // (nb <= 64) or blocked with shared-memory panels.
 template <int NB>
 struct StagedOps {
-  static constexpr bool kMixed = false;
+  static constexpr bool kMixed = false, kGroup = false;
   static constexpr int kMinBlocks = 2;
   static size_t smem_bytes(int) { return StagedCfg<NB>::SMEM; }
   SmemInv& inv;
   double2* dyn;
   double2* X;
   double2* Rt;
-  __device__ StagedOps(SmemInv& i, double2* dyn_, double2* slot_inv, double2* slot_rt, int)
-      : inv(i), dyn(dyn_), X(StagedCfg<NB>::SMEM_INV ? dyn_ : slot_inv), Rt(slot_rt) {}
+  SoloGroup grp;
+  __device__ StagedOps(SmemInv& i, double2* dyn_, double2* slot_inv, double2* slot_rt, int, Group = Group{})
+      : inv(i), dyn(dyn_), X(NB <= 64 ? dyn_ : slot_inv), Rt(slot_rt) {}
   template <class Epi>
   __device__ void gemm(int, const double2* A, bool cA, const double2* B, bool cB, Epi&& epi) {
     gemm_staged<NB>(NB, NB, NB, A, NB, cA, B, NB, cB, dyn, epi);
   }
   __device__ int invert(int, double2* dst, double2* dst2) {
     // nb = 32: matrix in registers (4 elements a thread); nb = 64: in shared
-    // memory as one panel of the blocked form (the register form, 16
-    // elements a thread, measured slower)
-    if constexpr (NB == 32)
-      return gj_invert_reg<NB>(X, dst, dst2, inv, dyn + (size_t)NB * NB);
-    else if constexpr (StagedCfg<NB>::SMEM_INV)
-      return gj_invert_smem_blocked<NB>(X, dst, dst2, inv, dyn + (size_t)NB * NB);
-    else return gj_invert_blocked<NB>(X, Rt, dst, dst2, dyn, dyn, inv);
+    // memory as one panel (the register form, 16 elements a thread, measured
+    // slower); larger: panels.  The same arithmetic as TiledOps, so a task's
+    // results do not depend on how many CTAs share it.
+    if constexpr (NB == 32) return gj_invert_reg(grp, NB, X, dst, dst2, inv, dyn + (size_t)NB * NB);
+    else if constexpr (NB == 64) return gj_invert_panel<NB, NB, 0>(Group{}, NB, X, dst, dst2, inv, dyn + (size_t)NB * NB);
+    else if constexpr (NB == 128) return gj_invert_blocked<NB>(X, Rt, dst, dst2, dyn, dyn, inv);
+    else return gj_invert_tiled<NB, NB>(Group{}, NB, X, Rt, dst, dst2, dyn, inv);
   }
   // >= NB complex values of shared memory free between block operations
+  __device__ double2* scratch() const { return dyn; }
+};
+
+// The tiled operations of rgf_tiled.cuh: any nb that is a multiple of 8 (NC =
+// 0), and nb = NC where a cluster shares a task (the size at compile time is
+// worth 1.2x there: nb = 128 on 8 CTAs 35 against 42 ms for 12 energies).  Up
+// to nb = 64 the matrix to invert is assembled in shared memory (a product is
+// one tile there, so nothing loads stages over it), unless several CTAs
+// assemble it.
+template <int NC>
+struct TiledOps {
+  static constexpr bool kMixed = false, kGroup = true;
+  static constexpr int kMinBlocks = 2;
+  SmemInv& inv;
+  double2* dyn;
+  double2* X;
+  double2* Rt;
+  Group grp;
+  __device__ TiledOps(SmemInv& i, double2* dyn_, double2* slot_inv, double2* slot_rt, int n, Group g)
+      : inv(i), dyn(dyn_), X((NC ? NC : n) <= 64 && g.size == 1 ? dyn_ : slot_inv), Rt(slot_rt), grp(g) {}
+  template <class Epi>
+  __device__ void gemm(int n_, const double2* A, bool cA, const double2* B, bool cB, Epi&& epi) {
+    const int n = NC ? NC : n_;
+    gemm_tiles(grp, n, n, n, A, n, cA, B, n, cB, dyn, NoInit{}, epi, nullptr, AllCols{});
+  }
+  __device__ int invert(int n_, double2* dst, double2* dst2) {
+    const int n = NC ? NC : n_;
+    if (n <= 32) return gj_invert_reg(grp, n, X, dst, dst2, inv, dyn + 32 * 32);
+    if (n <= 64) {
+      if (grp.size == 1) return gj_invert_panel<64, NC, 0>(grp, n, X, dst, dst2, inv, dyn + (size_t)n * n);
+      return gj_invert_tiled<64, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
+    }
+    if (n <= 128) return gj_invert_tiled<128, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
+    return gj_invert_tiled<256, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
+  }
+  // >= nb complex values of shared memory free between block operations
   __device__ double2* scratch() const { return dyn; }
 };
 
@@ -131,15 +169,76 @@ struct Solver {
   int n, nx;
   size_t n2;
   int status = 0, n_gemm = 0, n_inv = 0;
+  // the CTAs of this task (kGroup: several may share it)
+  std::conditional_t<Ops::kGroup, Group, SoloGroup> grp;
+  int parity = 0;   // of sum2's exchange slots
 
   __device__ Solver(const KOpts& o_, int64_t nx_max_, Smem& sm_, Ops& ops_, double2* slot_,
                     int n_, int nx_)
       : o(o_), nx_max(nx_max_), sm(sm_), ops(ops_), X(ops_.X), slot(slot_), n(n_), nx(nx_),
-        n2((size_t)n_ * n_) {}
+        n2((size_t)n_ * n_) {
+    if constexpr (Ops::kGroup) grp = ops_.grp;
+  }
 
   __device__ double2* tmp(int k) const { return slot + 2 * nx_max * n2 + (size_t)k * n2; }
   __device__ double2* Gl(int l) const { return slot + (size_t)l * n2; }
   __device__ double2* Gln(int l) const { return slot + (nx_max + l) * n2; }
+
+  __device__ __forceinline__ void sync() const { grp.sync(); }
+  // the thread that writes a task's scalars
+  __device__ __forceinline__ bool lead() const { return threadIdx.x == 0 && grp.rank == 0; }
+  // body(i, j, idx) over every element of a block, shared by the group (one
+  // division a call, not one an element)
+  template <class F>
+  __device__ __forceinline__ void each(F&& body) const {
+    const int first = threadIdx.x + kThreads * grp.rank, stride = kThreads * grp.size, nn2 = n * n;
+    const int dj = stride / n, di = stride - dj * n;
+    int j = first / n, i = first - j * n;
+    for (int idx = first; idx < nn2; idx += stride) {
+      body(i, j, idx);
+      i += di;
+      j += dj;
+      if (i >= n) { i -= n; j++; }
+    }
+  }
+  // The same walk by every CTA of the group: traces are formed whole by each,
+  // in an order that does not depend on the group.
+  template <class F>
+  __device__ __forceinline__ void each_whole(F&& body) const {
+    const int dj = kThreads / n, di = kThreads - dj * n, nn2 = n * n;
+    int j = threadIdx.x / n, i = threadIdx.x - j * n;
+    for (int idx = threadIdx.x; idx < nn2; idx += kThreads) {
+      body(i, j, idx);
+      i += di;
+      j += dj;
+      if (i >= n) { i -= n; j++; }
+    }
+  }
+  __device__ __forceinline__ double2 whole_sum(double2 v) { return block_sum2(v, sm.red); }
+  // Sum over the group; every thread gets the same value (fixed order).  The
+  // CTAs' sums are exchanged through two sets of slots used in turn, so one
+  // barrier suffices: a slot is written again only after the next exchange's
+  // barrier, which every reader of this one has passed.
+  __device__ __forceinline__ double2 sum2(double2 v) {
+    const double2 s = block_sum2(v, sm.red);
+    if (grp.size == 1) return s;
+    if ((int)threadIdx.x < grp.size) {
+      uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.part[parity][grp.rank]);
+      asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(dst) : "r"((uint32_t)threadIdx.x));
+      asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(dst), "d"(s.x), "d"(s.y) : "memory");
+    }
+    sync();
+    double2 t = czero();
+    for (int r = 0; r < grp.size; r++) t = cadd(t, sm.part[parity][r]);
+    parity ^= 1;
+    return t;
+  }
+  // Tr[A B] (only the diagonal of the product is formed)
+  __device__ __forceinline__ double2 trace(const double2* A, const double2* B) {
+    double2 acc = czero();
+    each_whole([&](int i, int k, int idx) { acc = cadd(acc, cmul(A[idx], B[k + i * n])); });
+    return whole_sum(acc);
+  }
 
   // Mixed form only: the block operations of the device chain run in the
   // split-integer / refined form, Sancho-Rubio and its self-energies in FP64.
@@ -157,7 +256,7 @@ struct Solver {
   __device__ void gemm(const double2* A, bool cA, const double2* B, bool cB, Epi&& epi) {
     if (fp64_now()) n_gemm++;
     ops.gemm(n, A, cA, B, cB, epi);
-    __syncthreads();
+    sync();
   }
   // C = op(A) op(B)
   __device__ void gemm_store(const double2* A, bool cA, const double2* B, bool cB, double2* C,
@@ -245,18 +344,18 @@ struct Solver {
           l = make_double2(g.x * rs, g.y * rs);
           d -= l.x * l.x + l.y * l.y;
         }
-        L[tid + k * nn] = l;
+        if (grp.rank == 0) L[tid + k * nn] = l;
         lcol[tid] = tid == p ? czero() : l;  // row and column p are never read again
       }
       __syncthreads();
-      for_each_elem(n, [&](int i, int j, int idx) {
+      each([&](int i, int j, int idx) {
         const double2 a = lcol[i], b = lcol[j];
         if ((a.x == 0.0 && a.y == 0.0) || (b.x == 0.0 && b.y == 0.0)) return;
         G[idx] = csub(G[idx], cmul(a, cconj(b)));
       });
-      __syncthreads();
+      sync();
     }
-    for (int e = tid; e < (nn - k) * nn; e += kThreads) L[(size_t)k * nn + e] = czero();
+    for (int e = tid + kThreads * grp.rank; e < (nn - k) * nn; e += kThreads * grp.size) L[(size_t)k * nn + e] = czero();
     double dmin = (own && !used) ? d : 0.0;
 #pragma unroll
     for (int o = 16; o; o >>= 1) dmin = fmin(dmin, __shfl_xor_sync(0xffffffffu, dmin, o));
@@ -265,7 +364,7 @@ struct Solver {
     dmin = 0.0;
 #pragma unroll
     for (int w = 0; w < kWarps; w++) dmin = fmin(dmin, sm.red.v[w]);
-    __syncthreads();
+    sync();
     return !(dmin < -neg_tol);
   }
 
@@ -279,20 +378,20 @@ struct Solver {
     const double2 z = make_double2(E, o.eta_lead);
     double2 *H10 = tmp(T_H10A), *H10n = tmp(T_H10B), *H01 = tmp(T_H01A), *H01n = tmp(T_H01B);
     double2 *HBB = tmp(T_HBB), *HSS = tmp(T_HSS), *SA = tmp(T_SA), *SB = tmp(T_SB);
-    for_each_elem(n, [&](int i, int j, int idx) {
+    each([&](int i, int j, int idx) {
       HBB[idx] = H00[idx];
       HSS[idx] = H00[idx];
       const double2 a = src[idx], at = src[j + i * nn];
       H10[idx] = conj_src ? cconj(at) : a;
       H01[idx] = conj_src ? a : cconj(at);
     });
-    __syncthreads();
+    sync();
     int taken = 0;
     for (int it = 1; it <= o.sancho_nmax; it++) {
       taken = it;
       // A = inv(z*S00 - H_BB)
-      for_each_elem(n, [&](int i, int j, int idx) { X[idx] = zs_minus(z, S00, i, j, idx, HBB[idx]); });
-      __syncthreads();
+      each([&](int i, int j, int idx) { X[idx] = zs_minus(z, S00, i, j, idx, HBB[idx]); });
+      sync();
       invert_X(SA);
       gemm_store(SA, false, H10, false, SB);                         // B = A H_10
       gemm(H01, false, SB, false, [&](int i, int j, double2 v) {     // C = H_01 B; H_SS += C; H_BB += C
@@ -313,18 +412,18 @@ struct Solver {
       });
       double2* t1 = H10; H10 = H10n; H10n = t1;
       double2* t2 = H01; H01 = H01n; H01n = t2;
-      const double err = block_sum2(make_double2(err_local, 0.0), sm.red).x;
+      const double err = sum2(make_double2(err_local, 0.0)).x;
       if (fabs(err) < o.sancho_tol) break;
       if (it == o.sancho_nmax) {
-        for_each_elem(n, [&](int, int, int idx) { HSS[idx] = H00[idx]; HBB[idx] = H00[idx]; });
-        __syncthreads();
+        each([&](int, int, int idx) { HSS[idx] = H00[idx]; HBB[idx] = H00[idx]; });
+        sync();
         status |= RGF_ST_SANCHO_NC;
         taken = o.sancho_nmax + 1;
       }
     }
     // G00 = inv(z*S00 - H_SS); the reference's GBB inverse is unused and skipped
-    for_each_elem(n, [&](int i, int j, int idx) { X[idx] = zs_minus(z, S00, i, j, idx, HSS[idx]); });
-    __syncthreads();
+    each([&](int i, int j, int idx) { X[idx] = zs_minus(z, S00, i, j, idx, HSS[idx]); });
+    sync();
     invert_X(GS);
     return taken;
   }
@@ -332,11 +431,11 @@ struct Solver {
   // Publishes that the outputs of the last `count` blocks are in memory for
   // a reader outside the GPU (the pipelined host copies): every thread's
   // stores are made visible system-wide, then one thread sets the counter.
-  __device__ static void publish(int32_t* progress, int count) {
+  __device__ void publish(int32_t* progress, int count) const {
     if (!progress) return;
     __threadfence_system();
-    __syncthreads();
-    if (threadIdx.x == 0) *(volatile int32_t*)progress = count;
+    sync();
+    if (lead()) *(volatile int32_t*)progress = count;
   }
 
   __device__ void run(const DTask& tk, const DDev& dv, DInfo* info, int32_t* progress = nullptr) {
@@ -369,10 +468,10 @@ struct Solver {
     double2* H00 = tmp(T_H00);
     {
       const double2* sr0 = scat(sr, 0, T_SRS);
-      for_each_elem(n, [&](int, int, int idx) {
+      each([&](int, int, int idx) {
         H00[idx] = sr0 ? cadd(Hii[idx], sr0[idx]) : Hii[idx];
       });
-      __syncthreads();
+      sync();
     }
     const double2* H10 = blk(H1i, 0);
     const int itL = sancho(E, H00, H10, true, tmp(T_GS), S_l(0));
@@ -385,7 +484,7 @@ struct Solver {
       double2* gam = tmp(T_F3);
       const double2* sl0 = scat(sl, 0, T_SLS);
       const double2* S0 = S_l(0);
-      for_each_elem(n, [&](int i, int j, int idx) {
+      each([&](int i, int j, int idx) {
         const double2 s = sigmal[idx], st = cconj(sigmal[j + i * nn]);
         const double2 w = csub(s, st);
         if (ballistic) {
@@ -397,7 +496,7 @@ struct Solver {
         }
         X[idx] = csub(zs_minus(z, S0, i, j, idx, H00[idx]), s);      // A = z S00 - H00 - sigmal
       });
-      __syncthreads();
+      sync();
     }
     set_mixed(true);   // the device chain (mixed form)
     invert_X(Gl(0));
@@ -411,10 +510,10 @@ struct Solver {
     // general recursion runs.
     const bool lowrank = ballistic && chol_psd(tmp(T_F3), tmp(T_SIG));
     if (ballistic && !lowrank) {
-      for_each_elem(n, [&](int i, int j, int idx) {
+      each([&](int i, int j, int idx) {
         tmp(T_SIG)[idx] = cscale(csub(sigmal[idx], cconj(sigmal[j + i * nn])), -fl);
       });
-      __syncthreads();
+      sync();
     }
     if (lowrank) {
       gemm_store(Gl(0), false, tmp(T_SIG), false, GN1buf[gsel]);   // V_1 = g_1 L
@@ -471,10 +570,10 @@ struct Solver {
       const int l = nx - 1;
       const double2* Hl = blk(Hii, l);
       const double2* srl = scat(sr, l, T_SRS);
-      for_each_elem(n, [&](int, int, int idx) {
+      each([&](int, int, int idx) {
         H00[idx] = srl ? cadd(Hl[idx], srl[idx]) : Hl[idx];
       });
-      __syncthreads();
+      sync();
     }
     const double2* H = blk(H1i, nx - 1);
     set_mixed(false);  // the right lead in FP64
@@ -528,7 +627,7 @@ struct Solver {
     {
       // tr = -Re sum_i [ (A1 Gp)_ii - (A2 Gn)_ii ],  A1 = -(sR - sR^H) fR, A2 = -(sR - sR^H)(fR - 1)
       double acc = 0.0;
-      for_each_elem(n, [&](int i, int k, int idx) {
+      each_whole([&](int i, int k, int idx) {
         const double2 gam = cscale(csub(sigmar[idx], cconj(sigmar[k + i * nn])), -1.0);
         const int ki = k + i * nn;
         const double2 gn = Gn[ki];
@@ -537,33 +636,33 @@ struct Solver {
         const double2 c = cmul(cscale(gam, fR - 1.0), gn);
         acc += b.x - c.x;
       });
-      const double s = block_sum2(make_double2(acc, 0.0), sm.red).x;
-      if (tk.tr && threadIdx.x == 0) *tk.tr = -s;
+      const double s = whole_sum(make_double2(acc, 0.0)).x;
+      if (tk.tr && lead()) *tk.tr = -s;
     }
     if (want_T) {
       gemm_store(H, false, GN1, false, tmp(T_X1));                  // H_{N,N-1} g^L_{N-1,1} (L)
       gemm_store(G00, false, tmp(T_X1), false, tmp(T_X2));          // G_{N1} (L)
-      for_each_elem(n, [&](int i, int j, int idx) {                 // Gamma = i (Sigma - Sigma^H)
+      each([&](int i, int j, int idx) {                 // Gamma = i (Sigma - Sigma^H)
         const double2 dl = csub(sigmal[idx], cconj(sigmal[j + i * nn]));
         const double2 dr = csub(sigmar[idx], cconj(sigmar[j + i * nn]));
         tmp(T_GAML)[idx] = make_double2(-dl.y, dl.x);
         tmp(T_GAMR)[idx] = make_double2(-dr.y, dr.x);
       });
-      __syncthreads();
+      sync();
       gemm_store(tmp(T_GAMR), false, tmp(T_X2), false, tmp(T_Y));   // Gamma_R G_N1 (L)
       if (lowrank) {
         // X2 = G_N1 L: T = Tr[Gamma_R X2 X2^H] = sum_ij Re (Gamma_R X2)_ij conj(X2_ij)
         double acc = 0.0;
-        for_each_elem(n, [&](int, int, int idx) {
+        each_whole([&](int, int, int idx) {
           const double2 y = tmp(T_Y)[idx], x = tmp(T_X2)[idx];
           acc += y.x * x.x + y.y * x.y;
         });
-        const double tt = block_sum2(make_double2(acc, 0.0), sm.red).x;
-        if (threadIdx.x == 0) *tk.T = tt;
+        const double tt = whole_sum(make_double2(acc, 0.0)).x;
+        if (lead()) *tk.T = tt;
       } else {
         gemm_store(tmp(T_GAML), false, tmp(T_X2), true, tmp(T_Z));  // Gamma_L G_N1^H
-        const double2 tt = trace_prod(n, tmp(T_Y), tmp(T_Z), sm.red);
-        if (threadIdx.x == 0) *tk.T = tt.x;
+        const double2 tt = trace(tmp(T_Y), tmp(T_Z));
+        if (lead()) *tk.T = tt.x;
       }
     }
 
@@ -577,7 +676,7 @@ struct Solver {
     // no scattering Sigma^<: every Gl< is anti-Hermitian by construction
     // (g Sigma^<_lead g^H and g H Gl< H^H g^H with anti-Hermitian factors)
     if (need_cur)
-      for_each_elem(n, [&](int, int, int idx) { blk2(tk.cur, nx - 1)[idx] = 0.0; });
+      each([&](int, int, int idx) { blk2(tk.cur, nx - 1)[idx] = 0.0; });
     if (need_back) publish(progress, 1);   // block nx-1: from the right closure
     for (int l = need_back ? nx - 2 : -1; l >= 0; l--) {
       const double2* Hb = blk(H1i, o.consistent ? l + 1 : l);
@@ -652,7 +751,7 @@ struct Solver {
         double2* nd = tk.ndens ? wblk(tk.ndens, l) : nullptr;
         double2* pd = (tk.pdens && !cms) ? wblk(tk.pdens, l) : nullptr;
         if (ballistic || ld || nd || pd) {
-          for_each_elem(n, [&](int i, int j, int idx) {
+          each([&](int i, int j, int idx) {
             const double2 g = G00n[idx];
             double2 w = Gnn[idx];
             if (ballistic) {
@@ -663,7 +762,7 @@ struct Solver {
             if (nd) nd[idx] = w;
             if (pd) pd[idx] = cadd(w, csub(g, cconj(G00n[j + i * nn])));
           });
-          __syncthreads();
+          sync();
         }
       }
       if (cms && (tk.pdens || tk.GGi1)) {
@@ -686,7 +785,7 @@ struct Solver {
     if (tk.tre) {
       const double fl2 = fermi((E - mul) / (o.boltz * tempr));   // TEMPr: as the reference (:4152)
       double acc = 0.0;
-      for_each_elem(n, [&](int i, int k, int idx) {
+      each_whole([&](int i, int k, int idx) {
         const double2 gam = cscale(csub(sigmal[idx], cconj(sigmal[k + i * nn])), -1.0);
         const int ki = k + i * nn;
         const double2 gn = Gn[ki];
@@ -695,17 +794,17 @@ struct Solver {
         const double2 c = cmul(cscale(gam, fl2 - 1.0), gn);
         acc += b.x - c.x;
       });
-      const double s = block_sum2(make_double2(acc, 0.0), sm.red).x;
-      if (threadIdx.x == 0) *tk.tre = s;
+      const double s = whole_sum(make_double2(acc, 0.0)).x;
+      if (lead()) *tk.tre = s;
     }
-    if (info && threadIdx.x == 0) {
+    if (info && lead()) {
       info->status = status;
       info->sancho_iters_left = itL;
       info->sancho_iters_right = itR;
       info->n_gemm = n_gemm;
       info->n_inv = n_inv;
     }
-    __syncthreads();
+    sync();
   }
 
 
@@ -731,7 +830,7 @@ struct Solver {
         dsum += fabs(v.x) + fabs(v.y);
         xsum += fabs(x.x) + fabs(x.y);
       });
-      const double2 sums = block_sum2(make_double2(dsum, xsum), sm.red);
+      const double2 sums = sum2(make_double2(dsum, xsum));
       if (!(sums.x > 1e-17 * sums.y)) break;
       gemm_store(P, false, P, false, P2);
       gemm_store(R, false, R, false, R2);
@@ -792,8 +891,8 @@ struct Solver {
         X[idx] = cadd(tmp(T_SA)[idx], v);
       });
       invert_X(Gl(l));
-      for_each_elem(n, [&](int, int, int idx) { tmp(T_F4)[idx] = csub(blk(Vii, l)[idx], tmp(T_F3)[idx]); });
-      __syncthreads();
+      each([&](int, int, int idx) { tmp(T_F4)[idx] = csub(blk(Vii, l)[idx], tmp(T_F3)[idx]); });
+      sync();
       gemm_store(Gl(l), false, tmp(T_F4), false, Gln(l));                         // Wlr_l
     }
     // ---- left-to-right: WR, Wo; W^< and W^> block by block
@@ -805,12 +904,12 @@ struct Solver {
     for (int l = 0; l < nx; l++) {
       double2* wr_out = wblk(tk.WR, l);
       if (l == 0) {
-        for_each_elem(n, [&](int, int, int idx) {
+        each([&](int, int, int idx) {
           const double2 w = Gln(0)[idx];
           WRc[idx] = w;
           wr_out[idx] = w;
         });
-        __syncthreads();
+        sync();
       } else {
         gemm_store(Gl(l), false, M1p, false, tmp(T_F1));                          // xlr_l M_{l,l-1}
         gemm(tmp(T_F1), false, Wop, false, [&](int i, int j, double2 v) {
@@ -826,8 +925,8 @@ struct Solver {
           M1c[i + j * nn] = m;
           M1T[j + i * nn] = m;
         });
-        for_each_elem(n, [&](int i, int j, int idx) { xT[j + i * nn] = Gl(l + 1)[idx]; });
-        __syncthreads();
+        each([&](int i, int j, int idx) { xT[j + i * nn] = Gl(l + 1)[idx]; });
+        sync();
         gemm(WRc, false, M1T, false, [&](int i, int j, double2 v) {               // C = V1i^T - WR M1i^T
           const int idx = i + j * nn;
           tmp(T_F2)[idx] = csub(blk(V1i, l)[j + i * nn], v);
@@ -869,14 +968,14 @@ struct Solver {
       t = Wic; Wic = Wip; Wip = t;
       t = NWTc; NWTc = NWTp; NWTp = t;
     }
-    if (info && threadIdx.x == 0) {
+    if (info && lead()) {
       info->status = status;
       info->sancho_iters_left = 0;
       info->sancho_iters_right = 0;
       info->n_gemm = n_gemm;
       info->n_inv = n_inv;
     }
-    __syncthreads();
+    sync();
   }
 
   __device__ void run_adjoint(const DAdj& tk, const DDev& dv, DInfo* info) {
@@ -898,8 +997,8 @@ struct Solver {
     auto sgc = [&](int q) { return Gln(cko + q); };
     double2* H00 = tmp(T_H00);
     // ---- left lead
-    for_each_elem(n, [&](int, int, int idx) { H00[idx] = Hii[idx]; });
-    __syncthreads();
+    each([&](int, int, int idx) { H00[idx] = Hii[idx]; });
+    sync();
     const int itL = sancho(E, H00, blk(H1i, 0), true, tmp(T_GS));
     double2* sigmal = tmp(T_SIGL);
     gemm_store(blk(H1i, 0), false, tmp(T_GS), false, tmp(T_F1));
@@ -915,26 +1014,26 @@ struct Solver {
     double2* cprev = tmp(T_GN1B);
     auto store_state = [&](int l, const double2* g, const double2* c) {
       if (nseg == 1) {
-        if (g != sgg(l)) for_each_elem(n, [&](int, int, int idx) { sgg(l)[idx] = g[idx]; sgc(l)[idx] = c[idx]; });
-        else for_each_elem(n, [&](int, int, int idx) { sgc(l)[idx] = c[idx]; });
-        __syncthreads();
+        if (g != sgg(l)) each([&](int, int, int idx) { sgg(l)[idx] = g[idx]; sgc(l)[idx] = c[idx]; });
+        else each([&](int, int, int idx) { sgc(l)[idx] = c[idx]; });
+        sync();
       } else if (l % S == 0) {
-        for_each_elem(n, [&](int, int, int idx) { ckg(l / S)[idx] = g[idx]; ckc(l / S)[idx] = c[idx]; });
-        __syncthreads();
+        each([&](int, int, int idx) { ckg(l / S)[idx] = g[idx]; ckc(l / S)[idx] = c[idx]; });
+        sync();
       }
     };
     // g_0
-    for_each_elem(n, [&](int i, int j, int idx) {
+    each([&](int i, int j, int idx) {
       const double2 h = Hii[idx];
       const double2 a = (i == j) ? make_double2(z.x - h.x, z.y - h.y) : make_double2(-h.x, -h.y);
       X[idx] = csub(a, sigmal[idx]);
     });
-    __syncthreads();
+    sync();
     double2* g0 = nseg == 1 ? sgg(0) : gprev;
     invert_X(g0);
     store_state(0, g0, g0);
-    if (nseg > 1) for_each_elem(n, [&](int, int, int idx) { cprev[idx] = g0[idx]; });
-    __syncthreads();
+    if (nseg > 1) each([&](int, int, int idx) { cprev[idx] = g0[idx]; });
+    sync();
     const double2* gl = g0;
     const double2* cl = nseg == 1 ? sgc(0) : cprev;
     // forward step from (g_{l-1}, c_{l-1}) to (g_l, c_l) into (gout, cout)
@@ -962,16 +1061,16 @@ struct Solver {
         double2* cn = tmp(T_G00B);
         fwd_step(l, gprev, cprev, gn, cn);
         store_state(l, gn, cn);
-        for_each_elem(n, [&](int, int, int idx) { gprev[idx] = gn[idx]; cprev[idx] = cn[idx]; });
-        __syncthreads();
+        each([&](int, int, int idx) { gprev[idx] = gn[idx]; cprev[idx] = cn[idx]; });
+        sync();
         gl = gprev;
         cl = cprev;
       }
     }
     // ---- right lead, G_NN, X = G_{N1}, T, W
     const double2* Hr = blk(H1i, nx - 1);
-    for_each_elem(n, [&](int, int, int idx) { H00[idx] = blk(Hii, nx - 1)[idx]; });
-    __syncthreads();
+    each([&](int, int, int idx) { H00[idx] = blk(Hii, nx - 1)[idx]; });
+    sync();
     const int itR = sancho(E, H00, Hr, false, tmp(T_GS));
     double2* sigmar = tmp(T_SIGR);
     gemm_store(Hr, true, tmp(T_GS), false, tmp(T_F1));
@@ -997,7 +1096,7 @@ struct Solver {
     double2* gamR = tmp(T_GAMR);
     double2* dgL = tmp(T_H10B);
     double2* dgR = tmp(T_H01A);
-    for_each_elem(n, [&](int i, int j, int idx) {
+    each([&](int i, int j, int idx) {
       const double2 dl = csub(sigmal[idx], cconj(sigmal[j + i * nn]));
       const double2 dr = csub(sigmar[idx], cconj(sigmar[j + i * nn]));
       gamL[idx] = make_double2(-dl.y, dl.x);
@@ -1007,7 +1106,7 @@ struct Solver {
       dgL[idx] = make_double2(-el.y, el.x);
       dgR[idx] = make_double2(-er.y, er.x);
     });
-    __syncthreads();
+    sync();
     double2* W = tmp(T_SIG);
     gemm_store(gamL, false, XN1, true, tmp(T_F1));                    // Gamma_L X^H
     gemm_store(tmp(T_F1), false, gamR, false, W);                     // W = Gamma_L X^H Gamma_R
@@ -1015,7 +1114,7 @@ struct Solver {
     gemm_store(gamR, false, XN1, false, tmp(T_F1));                   // Gamma_R X
     gemm_store(XN1, false, gamL, false, tmp(T_F2));                   // X Gamma_L
     gemm_store(tmp(T_F2), false, XN1, true, XGX);                     // X Gamma_L X^H
-    const double T = trace_prod(n, gamR, XGX, sm.red).x;
+    const double T = trace(gamR, XGX).x;
     // lead terms: Tr[Gamma_R X dGamma_L X^H] and Tr[dGamma_R X Gamma_L X^H]
     gemm_store(tmp(T_F1), false, dgL, false, tmp(T_F2));              // Gamma_R X dGamma_L
     gemm_store(tmp(T_F2), false, XN1, true, tmp(T_F4));
@@ -1023,27 +1122,27 @@ struct Solver {
     {
       double acc = 0.0;
       for (int i = threadIdx.x; i < n; i += kThreads) acc += tmp(T_F4)[i + i * nn].x;
-      leadL = block_sum2(make_double2(acc, 0.0), sm.red).x;
+      leadL = whole_sum(make_double2(acc, 0.0)).x;
     }
-    leadR = trace_prod(n, dgR, XGX, sm.red).x;
+    leadR = trace(dgR, XGX).x;
     // ---- reverse sweep
     double2 *r1 = tmp(T_Q1), *r0 = tmp(T_Q2), *k1 = tmp(T_Q3), *k0 = tmp(T_GNA);
     double2 *y1 = tmp(T_H01B), *y0 = tmp(T_HSS), *tA = tmp(T_F1), *tB = tmp(T_F2);
     // l = nx-1: r = G_NN, k = X
-    for_each_elem(n, [&](int, int, int idx) { r1[idx] = GNN[idx]; k1[idx] = XN1[idx]; });
-    __syncthreads();
+    each([&](int, int, int idx) { r1[idx] = GNN[idx]; k1[idx] = XN1[idx]; });
+    sync();
     gemm_store(W, false, r1, false, y1);                              // Y = W r
-    double gN = 2.0 * trace_prod(n, k1, y1, sm.red).x;
+    double gN = 2.0 * trace(k1, y1).x;
     // right lead term 2 Re Tr[W r_{N-1} S'_R X]
     gemm_store(y1, false, dSR, false, tA);
-    gN += 2.0 * trace_prod(n, tA, XN1, sm.red).x + leadR;
-    if (threadIdx.x == 0) tk.dTdV[nx - 1] = gN;
+    gN += 2.0 * trace(tA, XN1).x + leadR;
+    if (lead()) tk.dTdV[nx - 1] = gN;
     double ds = 0.0;
     for (int sg = nseg - 1; sg >= 0; sg--) {
       const int l0 = sg * S, l1 = (l0 + S < nl) ? l0 + S : nl;
       if (nseg > 1) {  // recompute the segment from its checkpoint
-        for_each_elem(n, [&](int, int, int idx) { sgg(0)[idx] = ckg(sg)[idx]; sgc(0)[idx] = ckc(sg)[idx]; });
-        __syncthreads();
+        each([&](int, int, int idx) { sgg(0)[idx] = ckg(sg)[idx]; sgc(0)[idx] = ckc(sg)[idx]; });
+        sync();
         for (int l = l0 + 1; l < l1; l++) fwd_step(l, sgg(l - 1 - l0), sgc(l - 1 - l0), sgg(l - l0), sgc(l - l0));
       }
       for (int l = l1 - 1; l >= l0; l--) {
@@ -1058,19 +1157,19 @@ struct Solver {
           k0[idx] = cadd(c[idx], v);
         });
         gemm_store(W, false, r0, false, y0);                          // Y_l = W r_l
-        double gl_ = 2.0 * trace_prod(n, k0, y0, sm.red).x;
+        double gl_ = 2.0 * trace(k0, y0).x;
         if (l == 0) {  // left lead: 2 Re Tr[W X S'_L k_0] + Tr[Gamma_R X dGamma_L X^H]
           gemm_store(W, false, XN1, false, tA);
           gemm_store(tA, false, dSL, false, tB);
-          gl_ += 2.0 * trace_prod(n, tB, k0, sm.red).x + leadL;
+          gl_ += 2.0 * trace(tB, k0).x + leadL;
         }
-        if (threadIdx.x == 0) tk.dTdV[l] = gl_;
+        if (lead()) tk.dTdV[l] = gl_;
         const int m = l + 1;                                          // coupling H_{m,m-1}
         if (m >= 1 && m <= nx - 2) {
           gemm_store(y1, false, Hn, false, tA);                       // Y_m H_{m,m-1}
-          double t1 = trace_prod(n, tA, k0, sm.red).x;
+          double t1 = trace(tA, k0).x;
           gemm_store(y0, false, Hn, true, tB);                        // Y_{m-1} H^H
-          t1 += trace_prod(n, tB, k1, sm.red).x;
+          t1 += trace(tB, k1).x;
           ds += 2.0 * t1;
         }
         double2* t;
@@ -1079,18 +1178,18 @@ struct Solver {
         t = y1; y1 = y0; y0 = t;
       }
     }
-    if (threadIdx.x == 0) {
+    if (lead()) {
       if (tk.T) *tk.T = T;
       if (tk.dTds) *tk.dTds = ds;
     }
-    if (info && threadIdx.x == 0) {
+    if (info && lead()) {
       info->status = status;
       info->sancho_iters_left = itL;
       info->sancho_iters_right = itR;
       info->n_gemm = n_gemm;
       info->n_inv = n_inv;
     }
-    __syncthreads();
+    sync();
   }
 
   __device__ double* blk2(double* base, int l) const { return base + (size_t)l * n2; }
@@ -1100,14 +1199,14 @@ struct Solver {
 // Gl[nx], Gln[nx] and the scratch blocks of this task's own nx and nb.
 template <class Ops>
 __device__ __forceinline__ void solve_task(const KParams& p, int64_t t, double2* slot, Smem& sm,
-                                           double2* dyn_smem) {
+                                           double2* dyn_smem, const Group& grp) {
   DInfo* info = p.info ? p.info + t : nullptr;
   const int dev = p.adj ? p.adj[t].dev : (p.wtasks ? p.wtasks[t].dev : p.tasks[t].dev);
   const DDev dv = p.devs[dev];
   const int n = (int)dv.nm;
   const size_t n2 = (size_t)n * n;
   double2* temps = slot + 2 * (size_t)dv.nx * n2;
-  Ops ops(sm.inv, dyn_smem, temps + (size_t)T_INV * n2, temps + (size_t)T_RT * n2, n);
+  Ops ops(sm.inv, dyn_smem, temps + (size_t)T_INV * n2, temps + (size_t)T_RT * n2, n, grp);
   Solver<Ops> s(p.o, dv.nx, sm, ops, slot, n, (int)dv.nx);
   if (p.adj) s.run_adjoint(p.adj[t], dv, info);
   else if (p.wtasks) s.run_w(p.wtasks[t], dv, info);

@@ -40,6 +40,9 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// dynamic shared memory of a CTA with two CTAs on an SM
+constexpr size_t kBlockSmem = 108 * 1024 + 512;
+
 template <int NB>
 struct StagedCfg {
   static constexpr int PM = NB < 64 ? NB : 64;   // output tile
@@ -51,31 +54,22 @@ struct StagedCfg {
   static constexpr int TM = WM / 8, TN = WN / 8;               // 8x8 subtiles per warp
   static constexpr int STAGE = 2 * KC * LDS;                   // complex values per stage (A + B)
   static constexpr int NSTAGE = 3;                             // cp.async pipeline depth (>= 2)
-  static constexpr int PW = NB >= 256 ? 16 : (NB >= 128 ? 48 : 32);  // inverse panel width (max)
-  static constexpr bool SMEM_INV = NB <= 64;                   // whole inverse in shared memory
-  // column pitch of the blocked inverse's shared panel (complex values): NB + 2
+  // the nb = 128 inverse's panel: width and column pitch (complex values; NB + 2
   // makes the rank-8 updates' fragment reads of 4 columns x 2 rows hit 8
-  // distinct 16-byte bank groups (pitch NB: 4-way conflicts)
-  static constexpr int LDP = SMEM_INV ? NB : NB + 2;
+  // distinct 16-byte bank groups)
+  static constexpr int PW = 48, LDP = NB + 2;
+  static_assert(NB != 128 || (size_t(LDP) * PW + PW + NB + 8 * PW) * sizeof(double2) <= kBlockSmem, "panel");
   static constexpr size_t GEMM_SMEM = size_t(NSTAGE) * STAGE * sizeof(double2);
-  // inverse: the matrix (nb <= 64) or one panel, then the row / column vectors
-  static constexpr size_t INV_MAT = SMEM_INV ? size_t(NB) * NB : size_t(LDP) * PW;
-  // inverse scratch after the matrix / panel, per form (complex values):
-  // blocked (nb >= 128): pivot row + multiplier column + 8 pivot rows of the
-  // panel's other columns, which also covers the sub-block elimination's
-  // scratch; register form (nb = 32); one-panel blocked form (nb = 64):
-  // 8 pivot rows of the other columns, or the sub-block scratch
-  static constexpr size_t SCR_SUB = 2 * size_t(NB) + 48 + size_t(NB) / 16;
-  static constexpr size_t SCR_PANEL = 2 * size_t(NB) + 8 * size_t(PW);
-  static constexpr size_t SCR_BLOCKED = SCR_PANEL > SCR_SUB ? SCR_PANEL : SCR_SUB;
-  static constexpr size_t SCR_REG = 6 * size_t(NB) + size_t(NB) / 8 + 8;
-  static constexpr size_t SCR_ONE = 8 * (size_t(NB) - 8) > SCR_SUB ? 8 * (size_t(NB) - 8) : SCR_SUB;
-  static constexpr size_t INV_SCR = !SMEM_INV ? SCR_BLOCKED : (NB == 32 ? SCR_REG : SCR_ONE);
-  static constexpr size_t INV_SMEM = (INV_MAT + INV_SCR) * sizeof(double2);
+  // inverse: nb = 32: the matrix as assembled, then the exchanged columns;
+  // nb = 64: the matrix, then the elimination's scratch; larger: a panel and
+  // the scratch (rgf_tiled.cuh's panel_width fills kBlockSmem)
+  static constexpr size_t INV_SMEM =
+      NB >= 128 ? kBlockSmem
+                : (size_t(NB) * NB + (NB == 32 ? 2 * 33 + 1 : 8 * (size_t(NB) - 8))) * sizeof(double2);
   static constexpr size_t SMEM = GEMM_SMEM > INV_SMEM ? GEMM_SMEM : INV_SMEM;
   // two CTAs per SM: 2 x (dynamic + static shared memory + 1 KB reserved)
   // within the SM's 228 KB
-  static_assert(SMEM <= 108 * 1024 + 512, "shared memory for two CTAs per SM");
+  static_assert(SMEM <= kBlockSmem, "shared memory for two CTAs per SM");
   static_assert(TM >= 1 && TN >= 1, "tile");
   static_assert(PM % (8 * WARPS_M) == 0 && PN % (8 * WARPS_N) == 0, "tile");
 };
@@ -191,129 +185,90 @@ __device__ __forceinline__ void gemm_staged(int M, int N, int K, const double2* 
   gemm_staged_init<NB>(M, N, K, A, lda, cA, B, ldb, cB, stage, NoInit{}, epi, brow);
 }
 
-// Gauss-Jordan inverse (partial pivoting) of the N x N block X (shared
-// memory; used for N = 32) with the matrix held in registers: thread tid owns row
-// tid % N and the CPT = N^2 / 256 consecutive columns of group tid / N.  Per
-// column k:
-//   (1) the owners of column k publish it and reduce the pivot key per warp
-//       (redux.sync), each forming the reciprocal of its entry meanwhile;
-//       barrier;
-//   (2) every thread combines the partials (largest key, first row on ties);
-//       the owners of row q publish the scaled pivot row r_j = x_qj / x_qk,
-//       the owners of row k publish row k; barrier;
-//   (3) every thread updates its elements, x_ij - f_i r_j (column k: -f_i r_k).
-// Key, tie and zero-pivot rules as gj_subblock.  At the end each thread
-// writes its elements to dst (and dst2) in the inverse's column order
-// (column c of the eliminated matrix is column coldst[c] of the inverse).
-// scr: 6 N + 4 N/32 + 8 complex values of shared scratch, double-buffered by
-// column parity.  Returns 1 (and zeros dst) on a zero pivot.
-template <int N>
-__device__ __noinline__ int gj_invert_reg(const double2* X, double2* dst, double2* dst2, SmemInv& s,
+// Gauss-Jordan inverse (partial pivoting) of the n x n block X, n <= 32, with
+// the matrix in registers: lane i of every warp owns row i, warp h the columns
+// 4 h .. 4 h + 3.  Rows are not interchanged (a used pivot row is marked), so
+// a warp gets the pivot row of its columns by shuffles and the CTA needs one
+// barrier a column: the warp that owns column k + 1 updates it, finds its
+// pivot (redux.sync) and publishes column, pivot row and reciprocal in the
+// buffer of the other parity before the barrier.  Bound by that chain: with
+// interchanges through shared memory and two barriers a column it took 61 k
+// cycles at nb = 32.
+//   pivot row q:  x_qj <- x_qj / x_qk (j = k: 1 / x_qk)
+//   other rows:   x_ij <- x_ij - x_ik x_qj / x_qk (j = k: - x_ik / x_qk)
+// With q_k the pivot row of step k, element (k, q_m) of the inverse is
+// x[q_k][m].  Pivot key, tie and zero-pivot rules as gj_subblock, ties broken
+// by the lower row.  scr: 2 x 33 complex values of shared scratch and two
+// words.  Every CTA of a group has the whole inverse and writes its share.
+// Returns 1 (and zeros dst) on a zero pivot.
+template <class G>
+__device__ __noinline__ int gj_invert_reg(G grp, int n, const double2* X, double2* dst, double2* dst2, SmemInv& s,
                                           double2* scr) {
-  constexpr int CPT = N * N / kThreads;  // columns per thread
-  constexpr int WPC = N / 32;            // warps owning one column
-  static_assert(CPT * kThreads == N * N && N % 32 == 0 && CPT >= 1, "register inverse layout");
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int i = tid % N, h = tid / N, j0 = h * CPT;
-  double2* fraw = scr;               // [2][N] column k before the step
-  double2* rr = fraw + 2 * N;        // [2][N] scaled pivot row
-  double2* rk = rr + 2 * N;          // [2][N] row k before the step
-  double2* pinvw = rk + 2 * N;       // [2][WPC] winners' reciprocals
-  unsigned* pk = reinterpret_cast<unsigned*>(pinvw + 2 * WPC);  // [2][WPC]
-  int* pi = reinterpret_cast<int*>(pk + 2 * WPC);               // [2][WPC]
+  constexpr int N = 32, CPT = N * N / kThreads;
+  const int lane = threadIdx.x & 31, h = threadIdx.x >> 5, j0 = h * CPT;
+  double2* col = scr;                          // [2][N] the published column
+  double2* piv = col + 2 * N;                  // [2] reciprocal of the pivot
+  int* prow = reinterpret_cast<int*>(piv + 2); // [2] pivot row, -1: zero pivot
   double2 x[CPT];
 #pragma unroll
-  for (int m = 0; m < CPT; m++) x[m] = X[i + (j0 + m) * N];
-  if (tid == 0) s.singular = 0;
-  for (int k = 0; k < N; k++) {
-    const int par = k & 1, hc = k / CPT, mc = k - hc * CPT;
-    if (h == hc) {
-      double2 v = x[0];
+  for (int m = 0; m < CPT; m++) x[m] = lane < n && j0 + m < n ? X[lane + (j0 + m) * n] : czero();
+  bool used = lane >= n;
+  int step = 0;                                // the step this row was the pivot of
+  auto publish = [&](double2 v, int k) {
+    const int par = k & 1;
+    col[par * N + lane] = v;
+    const double av = cabs1(v);
+    const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(av) >> 32);
+    const unsigned key = used ? 0u : (!(av == av) ? 1u : (av == 0.0 ? 2u : (hi > 1u ? hi : 1u) + 2u));
+    const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
+    const unsigned q = __reduce_min_sync(0xffffffffu, key == kmax ? (unsigned)lane : 0xffffffffu);
+    const double2 r = crecip(v);
+    if ((unsigned)lane == q) {
+      piv[par] = r;
+      prow[par] = kmax == 2u ? -1 : lane;
+      s.perm[k] = (int16_t)lane;
+    }
+  };
+  if (h == 0) publish(x[0], 0);
+  bool sing = false;
+  for (int k0 = 0; k0 < n; k0 += CPT) {
 #pragma unroll
-      for (int m = 1; m < CPT; m++)
-        if (m == mc) v = x[m];
-      fraw[par * N + i] = v;
-      const double av = cabs1(v);
-      unsigned key = 0u;
-      if (i >= k) {
-        const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(av) >> 32);
-        key = !(av == av) ? 1u : (av == 0.0 ? 2u : (hi > 1u ? hi : 1u) + 2u);
+    for (int c = 0; c < CPT; c++) {
+      const int k = k0 + c, par = c & 1;       // CPT is even: parity of k
+      if (k >= n) break;
+      __syncthreads();
+      const int q = prow[par];
+      if (q < 0) { sing = true; break; }       // uniform
+      const double2 pinv = piv[par], f = col[par * N + lane];
+      const bool own = h * CPT == k0;          // this warp's columns include k
+#pragma unroll
+      for (int m = 0; m < CPT; m++) {
+        const double2 xq = make_double2(__shfl_sync(0xffffffffu, x[m].x, q), __shfl_sync(0xffffffffu, x[m].y, q));
+        const bool kc = own && m == c;
+        const double2 r = kc ? pinv : cmul(xq, pinv);
+        const double2 b = kc ? czero() : x[m];
+        x[m] = lane == q ? r : make_double2(b.x - (f.x * r.x - f.y * r.y), b.y - (f.x * r.y + f.y * r.x));
       }
-      const double2 pv = crecip(v);
-      const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
-      const unsigned imin = __reduce_min_sync(0xffffffffu, key == kmax ? (unsigned)i : 0xffffffffu);
-      if ((unsigned)i == imin) {
-        const int w = warp - hc * WPC;
-        pk[par * WPC + w] = kmax;
-        pi[par * WPC + w] = i;
-        pinvw[par * WPC + w] = pv;
+      if (lane == q) {
+        used = true;
+        step = k;
       }
+      if (k + 1 < n && h == (k + 1) / CPT) publish(x[(c + 1) % CPT], k + 1);
     }
-    __syncthreads();
-    unsigned key = pk[par * WPC];
-    int q = pi[par * WPC], wq = 0;
-#pragma unroll
-    for (int w = 1; w < WPC; w++) {
-      const unsigned ek = pk[par * WPC + w];
-      const int ei = pi[par * WPC + w];
-      if (ek > key || (ek == key && ei < q)) { key = ek; q = ei; wq = w; }
-    }
-    if (tid == 0) {
-      if (key == 2u) s.singular = 1;
-      s.perm[k] = (int16_t)q;
-    }
-    if (i == q) {
-      const double2 pinv = pinvw[par * WPC + wq];
-#pragma unroll
-      for (int m = 0; m < CPT; m++) rr[par * N + j0 + m] = (j0 + m == k) ? pinv : cmul(x[m], pinv);
-    }
-    if (i == k) {
-#pragma unroll
-      for (int m = 0; m < CPT; m++) rk[par * N + j0 + m] = x[m];
-    }
-    __syncthreads();
-    const double2 f = (i == k) ? czero() : (i == q ? rk[par * N + k] : fraw[par * N + i]);
-#pragma unroll
-    for (int m = 0; m < CPT; m++) {
-      const int j = j0 + m;
-      const double2 r = rr[par * N + j];
-      if (i == k) {
-        x[m] = r;
-      } else {
-        const double2 base = (i == q) ? rk[par * N + j] : x[m];
-        const double2 xx = (j == k) ? czero() : base;
-        x[m] = make_double2(xx.x - (f.x * r.x - f.y * r.y), xx.y - (f.x * r.y + f.y * r.x));
-      }
-    }
+    if (sing) break;
   }
-  __syncthreads();
-  if (s.singular) {
-#pragma unroll
-    for (int m = 0; m < CPT; m++) {
-      dst[i + (j0 + m) * N] = czero();
-      if (dst2) dst2[i + (j0 + m) * N] = czero();
-    }
-    __syncthreads();
-    return 1;
-  }
-  if (tid == 0) {
-    for (int j = 0; j < N; j++) s.colsrc[j] = (int16_t)j;
-    for (int k = N - 1; k >= 0; k--) {
-      const int q = s.perm[k];
-      if (q != k) { const int16_t tmp = s.colsrc[k]; s.colsrc[k] = s.colsrc[q]; s.colsrc[q] = tmp; }
-    }
-  }
-  __syncthreads();
-  for (int j = tid; j < N; j += kThreads) s.coldst[s.colsrc[j]] = (int16_t)j;
   __syncthreads();
 #pragma unroll
   for (int m = 0; m < CPT; m++) {
-    const int o = i + s.coldst[j0 + m] * N;
-    dst[o] = x[m];
-    if (dst2) dst2[o] = x[m];
+    const int j = j0 + m;
+    if (lane >= n || j >= n || j % grp.size != grp.rank) continue;
+    const int o = sing ? lane + j * n : step + s.perm[j] * n;
+    const double2 v = sing ? czero() : x[m];
+    dst[o] = v;
+    if (dst2) dst2[o] = v;
   }
-  __syncthreads();
-  return 0;
+  grp.sync();
+  return sing ? 1 : 0;
 }
 
 // Gauss-Jordan elimination of the KB = 8 panel columns sb0.. (pivot rows
@@ -338,8 +293,9 @@ __device__ __noinline__ int gj_invert_reg(const double2* X, double2* dst, double
 // parity so one column's readers never race the next column's writers.
 // Returns with the sub-block written back to the panel and a barrier passed;
 // s.singular is set on a zero pivot.
-template <int NB, int LD = NB>
-__device__ __forceinline__ void gj_subblock(double2* panel, int PW, int p0, int sb0, double2* scr,
+// n <= NB rows; threads of rows from n on carry zeros that are never pivots.
+template <int NB>
+__device__ __forceinline__ void gj_subblock(int n, int LD, double2* panel, int PW, int p0, int sb0, double2* scr,
                                             int16_t* rmap, SmemInv& s) {
   constexpr int KB = 8;
   constexpr int CPT = KB * NB / kThreads;  // sub-block columns per thread
@@ -355,7 +311,7 @@ __device__ __forceinline__ void gj_subblock(double2* panel, int PW, int p0, int 
   int* pi = reinterpret_cast<int*>(pk + 2 * WPC);               // [2][WPC] rows
   double2 x[CPT];
 #pragma unroll
-  for (int m = 0; m < CPT; m++) x[m] = panel[i + (size_t)(sb0 + h * CPT + m) * LD];
+  for (int m = 0; m < CPT; m++) x[m] = i < n ? panel[i + (sb0 + h * CPT + m) * LD] : czero();
 #pragma unroll
   for (int cc = 0; cc < KB; cc++) {
     const int k = p0 + sb0 + cc, par = cc & 1;
@@ -365,7 +321,7 @@ __device__ __forceinline__ void gj_subblock(double2* panel, int PW, int p0, int 
       fraw[par * NB + i] = v;
       const double av = cabs1(v);
       unsigned key = 0u;
-      if (i >= k) {
+      if (i >= k && i < n) {
         const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(av) >> 32);
         key = !(av == av) ? 1u : (av == 0.0 ? 2u : (hi > 1u ? hi : 1u) + 2u);
       }
@@ -409,9 +365,9 @@ __device__ __forceinline__ void gj_subblock(double2* panel, int PW, int p0, int 
     if (q != k) {  // the panel's other columns: interchange rows k <-> q
       for (int j = tid; j < PW; j += kThreads) {
         if (j >= sb0 && j < sb0 + KB) continue;
-        const double2 a = panel[k + (size_t)j * LD];
-        panel[k + (size_t)j * LD] = panel[q + (size_t)j * LD];
-        panel[q + (size_t)j * LD] = a;
+        const double2 a = panel[k + j * LD];
+        panel[k + j * LD] = panel[q + j * LD];
+        panel[q + j * LD] = a;
       }
     }
     __syncthreads();
@@ -430,7 +386,8 @@ __device__ __forceinline__ void gj_subblock(double2* panel, int PW, int p0, int 
     }
   }
 #pragma unroll
-  for (int m = 0; m < CPT; m++) panel[i + (size_t)(sb0 + h * CPT + m) * LD] = x[m];
+  for (int m = 0; m < CPT; m++)
+    if (i < n) panel[i + (sb0 + h * CPT + m) * LD] = x[m];
   __syncthreads();
 }
 
@@ -441,8 +398,9 @@ __device__ __forceinline__ void gj_subblock(double2* panel, int PW, int p0, int 
 // on the FP64 tensor pipe: warp w owns rows 8 TMU w .. (TMU 8-row subtiles)
 // and walks the 8-column subtiles of the other columns; K = 8 is two m8n8k4
 // steps, U's fragments loaded once.  Ends with a barrier.
-template <int NB, int LD = NB>
-__device__ __forceinline__ void panel_rank8_update(double2* panel, int PW, int p0, int sb0, double2* rbuf) {
+template <int NB>
+__device__ __forceinline__ void panel_rank8_update(int n, int LD, double2* panel, int PW, int p0, int sb0,
+                                                   double2* rbuf) {
   constexpr int KB = 8;
   const int tid = threadIdx.x;
   const int nrest = PW - KB;
@@ -450,7 +408,7 @@ __device__ __forceinline__ void panel_rank8_update(double2* panel, int PW, int p
   for (int e = tid; e < KB * nrest; e += kThreads) {
     const int t = e % KB, jr = e / KB;
     const int j = jr < sb0 ? jr : jr + KB;
-    rbuf[t + jr * KB] = panel[(p0 + sb0 + t) + (size_t)j * LD];
+    rbuf[t + jr * KB] = panel[(p0 + sb0 + t) + j * LD];
   }
   __syncthreads();
   constexpr int TMU = NB / (8 * (kThreads / 32));
@@ -461,8 +419,9 @@ __device__ __forceinline__ void panel_rank8_update(double2* panel, int PW, int p
 #pragma unroll
   for (int ks = 0; ks < 2; ks++)
 #pragma unroll
-    for (int a = 0; a < TMU; a++) av[ks][a] = panel[(wm + 8 * a + g) + (size_t)(sb0 + 4 * ks + t4) * LD];
-  for (int b = 0; b < nrest / 8; b++) {
+    for (int a = 0; a < TMU; a++)
+      av[ks][a] = wm + 8 * a < n ? panel[(wm + 8 * a + g) + (sb0 + 4 * ks + t4) * LD] : czero();
+  for (int b = 0; wm < n && b < nrest / 8; b++) {
     double cr[TMU][1][2], ci[TMU][1][2];
 #pragma unroll
     for (int a = 0; a < TMU; a++) cr[a][0][0] = cr[a][0][1] = ci[a][0][0] = ci[a][0][1] = 0.0;
@@ -475,62 +434,16 @@ __device__ __forceinline__ void panel_rank8_update(double2* panel, int PW, int p
     for (int a = 0; a < TMU; a++)
 #pragma unroll
       for (int c = 0; c < 2; c++) {
+        if (TMU > 1 && wm + 8 * a >= n) continue;
         const int i = wm + 8 * a + g, jr = 8 * b + 2 * t4 + c;
         const int j = jr < sb0 ? jr : jr + KB;
         const bool prow = i >= p0 + sb0 && i < p0 + sb0 + KB;
-        const size_t o = i + (size_t)j * LD;
+        const int o = i + j * LD;
         const double2 x = prow ? czero() : panel[o];
         panel[o] = make_double2(x.x + cr[a][0][c], x.y + ci[a][0][c]);
       }
   }
   __syncthreads();
-}
-
-// Gauss-Jordan inverse (partial pivoting) of the NB x NB block X held whole
-// in shared memory (NB = 64): the blocked form of gj_invert_blocked with one
-// panel, i.e. 8-column sub-blocks eliminated with their elements in
-// registers (gj_subblock) and the other columns updated by rank-8 DMMA
-// products (panel_rank8_update); no trailing matrix.  Then dst[:, j] =
-// X[:, colsrc[j]] undoes the interchanges (and dst2 the same).  scr: shared
-// scratch of max(8 (NB - 8), 2 NB + 48 + NB / 16) complex values.  Returns 1
-// (and zeros dst) on a zero pivot.
-template <int NB>
-__device__ __noinline__ int gj_invert_smem_blocked(double2* X, double2* dst, double2* dst2, SmemInv& s,
-                                                   double2* scr) {
-  constexpr int KB = 8;
-  static_assert(NB % KB == 0, "whole sub-blocks");
-  const int tid = threadIdx.x;
-  if (tid == 0) s.singular = 0;
-  for (int i = tid; i < NB; i += kThreads) s.rmap[i] = (int16_t)i;
-  __syncthreads();
-  for (int sb0 = 0; sb0 < NB; sb0 += KB) {
-    gj_subblock<NB>(X, NB, 0, sb0, scr, s.rmap, s);
-    if (s.singular) break;
-    panel_rank8_update<NB>(X, NB, 0, sb0, scr);
-  }
-  if (s.singular) {
-    for_each_elem(NB, [&](int, int, int idx) {
-      dst[idx] = czero();
-      if (dst2) dst2[idx] = czero();
-    });
-    __syncthreads();
-    return 1;
-  }
-  if (tid == 0) {
-    for (int j = 0; j < NB; j++) s.colsrc[j] = (int16_t)j;
-    for (int k = NB - 1; k >= 0; k--) {
-      const int q = s.perm[k];
-      if (q != k) { const int16_t tmp = s.colsrc[k]; s.colsrc[k] = s.colsrc[q]; s.colsrc[q] = tmp; }
-    }
-  }
-  __syncthreads();
-  for_each_elem(NB, [&](int i, int j, int idx) {
-    const double2 v = X[i + s.colsrc[j] * NB];
-    dst[idx] = v;
-    if (dst2) dst2[idx] = v;
-  });
-  __syncthreads();
-  return 0;
 }
 
 // Blocked Gauss-Jordan inverse of the NB x NB block X0 (global memory, ld
@@ -543,7 +456,10 @@ __device__ __noinline__ int gj_invert_smem_blocked(double2* X, double2* dst, dou
 // (PW), multiplier column (NB) -- none of them is live during the update
 // GEMM, which reuses the same memory as its staging buffers.  The panel's row
 // map is read by that GEMM, so it lives in the static SmemInv.
-// Returns 1 (and zeros dst) on a zero pivot.
+// Returns 1 (and zeros dst) on a zero pivot.  nb = 128: the update with the
+// size at compile time, over all columns, beats the tiled one that leaves the
+// panel's own out (the benchmark's 296 energies 331 against 340 ms); the same
+// arithmetic.
 template <int NB>
 __device__ int gj_invert_blocked(double2* X0, double2* X1, double2* dst, double2* dst2,
                                  double2* smem, double2* stage, SmemInv& s) {
@@ -579,9 +495,9 @@ __device__ int gj_invert_blocked(double2* X0, double2* X1, double2* dst, double2
     static_assert(PWM % KB == 0 && (NB % PWM) % KB == 0, "panels of whole sub-blocks");
     double2* rbuf = fcol + NB;  // KB x PWM pivot rows of the other columns
     for (int sb0 = 0; sb0 < PW && !s.singular; sb0 += KB) {
-      gj_subblock<NB, C::LDP>(panel, PW, p0, sb0, rowk, rmap, s);
+      gj_subblock<NB>(NB, C::LDP, panel, PW, p0, sb0, rowk, rmap, s);
       if (s.singular) break;
-      panel_rank8_update<NB, C::LDP>(panel, PW, p0, sb0, rbuf);
+      panel_rank8_update<NB>(NB, C::LDP, panel, PW, p0, sb0, rbuf);
     }
     if (s.singular) break;
     // the last panel writes the inverse itself: its column j is column

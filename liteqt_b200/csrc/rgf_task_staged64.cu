@@ -5,8 +5,8 @@
 namespace rgf {
 
 __device__ __noinline__ void task_staged64(const KParams& p, int64_t t, double2* slot, Smem& sm,
-                                         double2* dyn) {
-  solve_task<StagedOps<64>>(p, t, slot, sm, dyn);
+                                         double2* dyn, Group grp) {
+  solve_task<StagedOps<64>>(p, t, slot, sm, dyn, grp);
 }
 
 }  // namespace rgf

@@ -57,7 +57,8 @@ EXPORTS = (
 )
 
 # kernel variant ids (rgf_variant_name)
-VARIANTS = ("staged32", "staged64", "staged128", "staged256", "generic1x1", "generic1x2", "generic2x2")
+VARIANTS = ("staged32", "staged64", "staged128", "staged256", "generic1x1", "generic1x2", "generic2x2",
+            "tiled")
 
 
 class RgfError(RuntimeError):
