@@ -1051,11 +1051,52 @@ static int launch_ctas_per_sm(const rgf_ctx* c, size_t smem, uint64_t nb_mask) {
 }
 
 // Geometry of a launch over n_tasks tasks of the block sizes in nb_mask: as
-// many CTAs as are resident at a time, one a task.
+// many CTAs as are resident at a time, one a task.  Fewer tasks than that
+// leave SMs idle while every task is a serial chain of block operations, so
+// the CTAs are then grouped in clusters of 2, 4 or 8 that share a task's
+// operations.  The rule goes by the largest block size, which dominates the
+// time (measured on 1 B200, nx = 10, G^R, G^<, G^>, ms with clusters of 1 / 2 /
+// 4 / 8, * = two CTAs on an SM):
+//   nb =  32,   1 energy:    1.9 /  2.7 /  2.7 /  2.7    cluster barriers cost more than the products
+//   nb =  64,  37 energies:  9.5 /  7.9 /  9.1*
+//   nb =  96,  37 energies: 42.9 / 26.4 / 25.5*          120 energies: 48.8 / 39.1*
+//   nb = 128,  18 energies: 55.0 / 34.9 / 23.1 / 25.7*   148 energies: 61.3 / 60.2*
+//   nb = 256,  18 energies:  402 /  227 /  128 /  120*   148 energies:  436 /  405*
+// So: no clusters up to nb = 32; otherwise the largest that leaves every CTA
+// an SM of its own; two CTAs an SM from nb = 192 on, and from nb = 80 on where
+// there would be no cluster otherwise.
 static SolverShape solver_shape(const rgf_ctx* c, size_t smem, uint64_t nb_mask, int64_t n_tasks) {
   SolverShape s;
-  s.groups = (int)std::min<int64_t>(c->sm_count * launch_ctas_per_sm(c, smem, nb_mask), n_tasks);
+  const int resident = c->sm_count * launch_ctas_per_sm(c, smem, nb_mask);
+  s.groups = (int)std::min<int64_t>(resident, n_tasks);
   s.smem = smem;
+  int nb = 0;
+  for (int i = 0; i < kVariantSlots; i++)
+    if ((nb_mask >> i) & 1) {
+      // a cluster runs the tiled operations, whose results are bit for bit
+      // those of the staged and tiled variants; a task of a register-direct
+      // variant would depend on what shares its launch
+      const int v = c->variant[i];
+      if (v == KV_GENERIC11 || v == KV_GENERIC12 || v == KV_GENERIC22) return s;
+      nb = 8 * i;
+    }
+  if (nb <= 32 || 2 * n_tasks > resident) return s;
+  smem = std::max(smem, variant_smem(KV_TILED, nb));
+  const size_t alone = std::max<size_t>(smem, 120 * 1024);   // more than two CTAs of an SM can have
+  auto fits = [&](int k, size_t bytes, int ctas) {
+    return n_tasks * k <= ctas && solver_max_clusters(bytes, k) >= n_tasks;
+  };
+  for (int k = 8; k > 1 && s.cluster == 1; k /= 2)
+    if (fits(k, alone, c->sm_count)) {
+      s.cluster = k;
+      s.smem = alone;
+    }
+  if (nb >= 192 || (nb >= 80 && s.cluster == 1))
+    for (int k = 8; k > s.cluster; k /= 2)
+      if (fits(k, smem, resident)) {
+        s.cluster = k;
+        s.smem = smem;
+      }
   return s;
 }
 
