@@ -334,12 +334,4 @@ __device__ __noinline__ static int gj_invert(int n, double2* X, double2* dst, do
   return 0;
 }
 
-// Re/Im of Tr[A * B] = sum_{i,k} A[i][k] B[k][i] (only the diagonal of the
-// product is formed).  opB_plus: B = B1 + (B2 - B2^H) when B2 is non-null.
-__device__ __forceinline__ double2 trace_prod(int n, const double2* A, const double2* B, SmemRed& r) {
-  double2 acc = czero();
-  for_each_elem(n, [&](int i, int k, int idx) { acc = cadd(acc, cmul(A[idx], B[k + i * n])); });
-  return block_sum2(acc, r);
-}
-
 }  // namespace rgf
