@@ -750,8 +750,11 @@ def run_gw(args):
     """GW-loop convolutions (green_rgf.f90:2944-3092) on device-resident
     arrays: 2x2 k-grid, nen = 512, nx = 10, nm = 16, ndiag = 3, seeded complex
     inputs.  One step = rgf_gw_polarization + rgf_gw_self_energy.  Roofline:
-    the FP64 pipe (4 complex multiply-adds = 32 flops per P summand, 5 = 40
-    per Sigma summand; summand counts of the reference's loops)."""
+    the FP64 pipe.  G is purely imaginary in these sums, so a P summand's four
+    products are real multiply-adds (8 flops) and a Sigma summand's four
+    (G^R W^< + G^R W^R as one) are two each (16 flops); Sigma's sums leave out
+    the four edge blocks that copies overwrite.  Summand counts of the
+    reference's loops otherwise."""
     import torch
     from liteqt_b200 import rgf
     nky, nkz, nen, nx, nm, ndiag = 2, 2, 512, 10, 16, 3
@@ -788,7 +791,8 @@ def run_gw(args):
                 ts.append(e[1].elapsed_time(e[2]))
     ctx.close()
     p_terms, s_terms = _gw_terms(nm, nx, nen, nk, ndiag)
-    fp, fs = 32.0 * p_terms, 40.0 * s_terms
+    s_terms = s_terms * (nx - 4) // nx
+    fp, fs = 8.0 * p_terms, 16.0 * s_terms
     mp, ms_ = float(np.mean(tp)), float(np.mean(ts))
     line = {"metric": "GW convolutions: polarization + self-energy steps/s", "value": 1e3 / (mp + ms_),
             "unit": "steps/s", "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
