@@ -214,7 +214,14 @@ struct Solver {
       if (i >= n) { i -= n; j++; }
     }
   }
-  __device__ __forceinline__ double2 whole_sum(double2 v) { return block_sum2(v, sm.red); }
+  // Every CTA has read the walk's operands whole when this returns, so the
+  // next operation may write them: without the barrier a CTA that runs ahead
+  // overwrites its share of an operand while another still reads it.
+  __device__ __forceinline__ double2 whole_sum(double2 v) {
+    const double2 s = block_sum2(v, sm.red);
+    if (grp.size > 1) sync();
+    return s;
+  }
   // Sum over the group; every thread gets the same value (fixed order).  The
   // CTAs' sums are exchanged through two sets of slots used in turn, so one
   // barrier suffices: a slot is written again only after the next exchange's
