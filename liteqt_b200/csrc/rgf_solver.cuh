@@ -315,7 +315,7 @@ struct Solver {
     amax = 0.0;
 #pragma unroll
     for (int w = 0; w < kWarps; w++) amax = fmax(amax, sm.red.v[w]);
-    __syncthreads();
+    sync();   // every CTA of the group has its diagonal before the first update of G
     const double neg_tol = (double)nn * 2.220446049250313e-16 * amax;
     int k = 0;
     for (; k < nn; k++) {
