@@ -2012,7 +2012,7 @@ extern "C" int rgf_plan_create(rgf_ctx* c, const rgf_device* devices, int32_t n_
   p.work = (double2*)pl->work.p;
   p.slot_elems = shape.slot;
   p.info = (DInfo*)pl->info.p;
-  solver_blocks_per_sm(geo.smem);  // raises the kernel's shared-memory limit before the capture
+  solver_blocks_per_sm(geo.smem);  // sets the kernel's shared-memory limit before the capture
   cudaStream_t cs = nullptr;
   RGF_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);

@@ -130,9 +130,18 @@ void set_default_variants(KParams& p) {
 
 int solver_threads() { return kThreads; }
 
+// The kernel's limit of dynamic shared memory belongs to the device, not to a
+// launch: it is always set to the same value, so a call on one host thread
+// never lowers it between another thread's setting and its launch.  The
+// launches and queries give their own size, which alone counts for occupancy.
+static cudaError_t allow_smem() {
+  constexpr int kLimit = 160 * 1024;
+  return cudaFuncSetAttribute(rgf_solver_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit);
+}
+
 int solver_blocks_per_sm(size_t smem) {
   int nblk = 0;
-  cudaFuncSetAttribute(rgf_solver_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem();
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nblk, rgf_solver_kernel, kThreads, smem) != cudaSuccess) {
     cudaGetLastError();
     return 1;
@@ -141,7 +150,7 @@ int solver_blocks_per_sm(size_t smem) {
 }
 
 int solver_max_clusters(size_t smem, int cluster) {
-  cudaFuncSetAttribute(rgf_solver_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  allow_smem();
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at = {};
   at.id = cudaLaunchAttributeClusterDimension;
@@ -162,7 +171,7 @@ int solver_max_clusters(size_t smem, int cluster) {
 
 cudaError_t launch_solver(const KParams& p, const SolverShape& s, cudaStream_t st, bool set_attr) {
   if (set_attr) {
-    cudaError_t e = cudaFuncSetAttribute(rgf_solver_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem);
+    const cudaError_t e = allow_smem();
     if (e != cudaSuccess) return e;
   }
   cudaLaunchConfig_t cfg = {};
