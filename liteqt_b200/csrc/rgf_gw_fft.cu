@@ -630,12 +630,16 @@ void k_transform(bool forward, const own::Six& in, const own::Three& out, const 
   RGF_K_CASE(4, 4);
 #undef RGF_K_CASE
   const size_t tile = (size_t)d.nk * own::kTileE * sizeof(double2);
+  // the kernels' limit belongs to the device: the same value from every
+  // thread, whatever its k-grid
+  constexpr size_t kMaxTile = (size_t)kAnyGridMaxK * own::kTileE * sizeof(double2);
   const unsigned ge = (unsigned)((d.nen + own::kTileE - 1) / own::kTileE);
   if (forward) {
-    cudaFuncSetAttribute(own::k_forward_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * tile));
+    cudaFuncSetAttribute(own::k_forward_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kMaxTile));
     own::k_forward_any<<<dim3(ge, (unsigned)nl, (unsigned)nops), 256, 2 * tile, st>>>(in, lines, nl, d, conj, ph, kb);
   } else {
-    cudaFuncSetAttribute(own::k_inverse_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * tile + tile / 2));
+    cudaFuncSetAttribute(own::k_inverse_any, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(2 * kMaxTile + kMaxTile / 2));
     own::k_inverse_any<<<dim3(ge, (unsigned)nl), 256, 2 * tile + tile / 2, st>>>(out, lines, nl, d, fix, ph, pb);
   }
 }

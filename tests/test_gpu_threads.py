@@ -1,6 +1,6 @@
 """GPU test of several host threads at work at the same time, each with its own
 context: calls of 1, 12 and 200 energies, block sizes with different shared
-memory.  Every call
+memory, and convolutions on k-grids with different shared memory.  Every call
 returns RGF_OK with the bits of a call made alone: nothing one call sets
 (limits of a kernel, which belong to the device) may disturb another."""
 import threading
@@ -67,6 +67,31 @@ def test_concurrent_solves(rgf, sizes):  # noqa: F811
                 assert torch.equal(v, want[nm][k][:nen]), (nm, nen, k)
         return run
     _together([job(sizes[i % len(sizes)], (1, 12, 1, 200)[(i // len(sizes)) % 4]) for i in range(16)])
+
+
+def test_concurrent_convolutions_on_different_grids(rgf):  # noqa: F811
+    import torch
+    nen, reps = 64, 40
+
+    def job(nkz):
+        def run(gate):
+            g = torch.Generator(device="cuda").manual_seed(nkz)
+            A = [torch.randn(4, 2, nkz, nen, dtype=torch.complex128, device="cuda", generator=g) for _ in range(5)]
+            out = [torch.zeros_like(A[0]) for _ in range(3)]
+            first = None
+            with rgf.Context(rgf.Options()) as ctx:
+                torch.cuda.synchronize()
+                gate.wait()
+                for _ in range(reps):
+                    ctx.gw_polarization_fft(*A, PL=out[0], PG=out[1], PR=out[2], nky=1, nkz=nkz, nm=2, ndiag=1,
+                                            first_ij=1, dEn=0.01, spindeg=2.0)
+                    if first is None:
+                        first = [o.clone() for o in out]
+                        torch.cuda.synchronize()
+            for a, b in zip(out, first):
+                assert torch.equal(a, b)
+        return run
+    _together([job(n) for n in (100, 3, 90, 5, 60, 7, 33, 9)])
 
 
 def test_plan_of_few_tasks_after_calls_with_other_limits(rgf):  # noqa: F811
