@@ -28,8 +28,8 @@
 //               the window; spectra that wait for a partner go to scratch of
 //               the resident CTAs (L2);
 //   k_inverse   the inverse k-grid transform of the windows with the phases.
-// Longer axes and k-grids whose tile does not fit take the form below it:
-// cuFFT's 3-D transforms (Z2Z, batched, stream-ordered) with separate packing,
+// Longer axes, and k-grids for which own_log finds it faster, take the form
+// below it: cuFFT's 3-D transforms (Z2Z, batched, stream-ordered) with separate packing,
 // product and window kernels.
 //
 // Arrays: the *_by_blocks layout (nen, nk, nx, nij) complex(8) on the device,
@@ -594,12 +594,30 @@ LineLaunch line_launch_for(int logm) {
   }
 }
 
-constexpr int64_t kAnyGridMaxK = 160;   // tile of the general k-grid kernels: 40 KB a k-point x 32 energies
-// log2 M, or 0 where the form does not apply
+// Where the own form pays (P + Sigma, 112 lines, ms, cuFFT form / own, 1 B200).
+// k-grids with both axes of 1, 2 or 4 points have their transform in registers
+// and win at every length (1 x 1: 130 energies 0.21 / 0.18, 2050 0.36 / 0.28,
+// 4096 0.51 / 0.34; 4 x 4: 0.53 / 0.22, 3.64 / 2.13, 7.1 / 2.8).  Other grids
+// sum their axes directly, at nky + nkz terms a value, against cuFFT:
+//   one axis:  130 energies, 1 x 7 0.36 / 0.26;  258, 1 x 3 0.34 / 0.30, 1 x 11
+//     0.50 / 0.52;  512, 1 x 3 0.37 / 0.38;  1026, 1 x 3 0.57 / 0.66;  2050,
+//     1 x 8 1.5 / 2.1;  512, 1 x 64 2.6 / 6.6
+//   two axes:  258, 3 x 3 0.60 / 0.44, 5 x 5 0.94 / 0.93;  512, 4 x 6 1.41 /
+//     1.18, 5 x 7 1.70 / 1.80;  514, 5 x 5 1.42 / 1.60;  2050, 3 x 3 2.0 / 2.7
+//     (energies padded to the next power of two);  1000, 4 x 6 2.7 / 2.2, 3 x 4
+//     1.38 / 1.35;  4096, 3 x 4 5.5 / 4.8
+// So: one axis up to 8 points and 256 energies; two axes up to 10 points
+// together, and 512 energies or a count that fills its power of two.
+bool any_grid_pays(const Dims& d, int64_t M) {
+  if (d.nky == 1 || d.nkz == 1) return d.nk <= 8 && M <= 256;
+  return d.nky + d.nkz <= 10 && (M <= 512 || 32 * d.nen > 31 * M);
+}
+// log2 M, or 0 where the cuFFT form is taken
 int own_log(const Dims& d) {
-  if (d.nk > kAnyGridMaxK) return 0;
+  auto small = [](int64_t n) { return n == 1 || n == 2 || n == 4; };
+  const bool registers = small(d.nky) && small(d.nkz);
   for (int l = own::kMinLog; l <= own::kMaxLog; l++)
-    if ((int64_t(1) << l) >= d.nen) return l;
+    if ((int64_t(1) << l) >= d.nen) return registers || any_grid_pays(d, int64_t(1) << l) ? l : 0;
   return 0;
 }
 
@@ -630,18 +648,11 @@ void k_transform(bool forward, const own::Six& in, const own::Three& out, const 
   RGF_K_CASE(4, 4);
 #undef RGF_K_CASE
   const size_t tile = (size_t)d.nk * own::kTileE * sizeof(double2);
-  // the kernels' limit belongs to the device: the same value from every
-  // thread, whatever its k-grid
-  constexpr size_t kMaxTile = (size_t)kAnyGridMaxK * own::kTileE * sizeof(double2);
   const unsigned ge = (unsigned)((d.nen + own::kTileE - 1) / own::kTileE);
-  if (forward) {
-    cudaFuncSetAttribute(own::k_forward_any, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * kMaxTile));
+  if (forward)   // at most 25 k-points: 32 KB of shared memory
     own::k_forward_any<<<dim3(ge, (unsigned)nl, (unsigned)nops), 256, 2 * tile, st>>>(in, lines, nl, d, conj, ph, kb);
-  } else {
-    cudaFuncSetAttribute(own::k_inverse_any, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)(2 * kMaxTile + kMaxTile / 2));
+  else
     own::k_inverse_any<<<dim3(ge, (unsigned)nl), 256, 2 * tile + tile / 2, st>>>(out, lines, nl, d, fix, ph, pb);
-  }
 }
 
 // ph: the nk phases, then the nky-th and nkz-th roots.

@@ -1,0 +1,30 @@
+"""GPU tests of the FFT convolutions on both sides of each limit between the
+library's own transforms and cuFFT's (counts of k-points and of energies),
+against the oracle; tolerance of test_gpu_gw_fft_sizes (FFT rounding on both
+sides)."""
+import numpy as np
+import pytest
+
+from oracle import gw_fft as F
+from test_gpu_gw_fft_sizes import TOL, rgf  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nky,nkz,nen", [(1, 8, 256), (1, 8, 258), (9, 1, 64), (1, 3, 256), (5, 5, 60), (5, 6, 60),
+                                         (3, 3, 512), (3, 3, 514), (3, 3, 992), (3, 3, 994), (2, 3, 1024), (1, 40, 34)])
+def test_fft_grids_on_both_routes(rgf, nky, nkz, nen):  # noqa: F811
+    import torch
+    nx, nk = 2, nky * nkz
+    rng = np.random.default_rng(nen + nk)
+    A = [rng.normal(size=(1, nx, nk, nen)) + 1j * rng.normal(size=(1, nx, nk, nen)) for _ in range(8)]
+    D = [torch.from_numpy(a).cuda() for a in A]
+    out = [torch.zeros_like(D[0]) for _ in range(6)]
+    grid = dict(nky=nky, nkz=nkz, nm=1, ndiag=0, first_ij=1, dEn=0.013)
+    with rgf.Context(rgf.Options()) as ctx:
+        ctx.gw_polarization_fft(*D[:5], PL=out[0], PG=out[1], PR=out[2], spindeg=2.0, **grid)
+        ctx.gw_self_energy_fft(*D[:3], *D[5:], SL=out[3], SG=out[4], SR=out[5], **grid)
+    want = list(F.gw_polarization_fft(*A[:5], nky, nkz, 1, 0, 1, 0.013, 2.0))
+    want += list(F.gw_self_energy_fft(*A[:3], *A[5:], nky, nkz, 1, 0, 1, 0.013))
+    for g, w in zip(out, want):
+        assert np.max(np.abs(g.cpu().numpy() - w)) <= TOL * np.max(np.abs(w))
