@@ -43,6 +43,7 @@
 #include <memory>
 #include <vector>
 
+#include "rgf_fft_cache.h"
 #include "rgf_fft_smem.cuh"
 #include "rgf_internal.h"
 
@@ -511,11 +512,9 @@ struct Plan {
 // iteration): the cuFFT plans of the last shape and the device scratch, so a
 // call neither re-plans nor re-allocates.  Freed with the context.
 struct FftCache {
-  int dev = -1;
-  int64_t nky = 0, nkz = 0, N = 0, chunk = 0, tail = 0;
+  rgf::FftKeys keys;                       // what scratch, full and part belong to
   std::unique_ptr<struct Plan> full, part;
   void* scratch = nullptr;
-  size_t bytes = 0;
   double2* roots[own::kMaxLog + 1] = {};   // own transforms: exp(-2 pi i n / 2M), n < M, then the twiddles
   int roots_dev = -1;
   cudaStream_t fill = nullptr;             // zeroes the elements outside the band beside the transforms
@@ -540,7 +539,7 @@ FftCache::~FftCache() {
   if (scratch) {
     int cur = 0;
     cudaGetDevice(&cur);
-    cudaSetDevice(dev);
+    cudaSetDevice(keys.scratch_dev);
     cudaFree(scratch);
     cudaSetDevice(cur);
   }
@@ -548,18 +547,18 @@ FftCache::~FftCache() {
 
 // cache->scratch of at least `need` bytes on device dev
 int reserve_scratch(FftCache* cache, int dev, size_t need, cudaStream_t st) {
-  if (cache->dev == dev && cache->bytes >= need) return RGF_OK;
+  if (cache->keys.scratch_fits(dev, need)) return RGF_OK;
   cudaError_t e = cudaStreamSynchronize(st);   // earlier calls may still use the old scratch
   if (cache->scratch) cudaFree(cache->scratch);
   cache->scratch = nullptr;
-  cache->bytes = 0;
+  cache->keys.set_scratch(dev, 0);
   if (e == cudaSuccess) e = cudaMalloc(&cache->scratch, need);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cache->scratch = nullptr;
     return fft_fail(RGF_E_NOMEM, "device scratch for the transforms");
   }
-  cache->bytes = need;
+  cache->keys.set_scratch(dev, need);
   return RGF_OK;
 }
 
@@ -676,7 +675,6 @@ int run_own(FftCache* cache, int dev, int mode, const Dims& d, int logm, const s
   const size_t scr = (size_t)ctas * L.group * 3 * M;
   int rc = reserve_scratch(cache, dev, sizeof(double2) * (per_line * chunk + scr + ph.size()) + sizeof(int64_t) * nl, st);
   if (rc) return rc;
-  cache->dev = dev;
   if (cache->roots_dev != dev) {
     for (double2*& r : cache->roots) {
       if (r) cudaFree(r);
@@ -852,8 +850,9 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
   const int rc = reserve_scratch(cache, dev, need, st);
   if (rc) return rc;
   const int64_t tail = nl % chunk;
-  if (cache->dev != dev || cache->nky != nky || cache->nkz != nkz || cache->N != d.N || cache->chunk != chunk ||
-      cache->tail != tail || !cache->full) {
+  const rgf::FftPlanKey key{dev, nky, nkz, d.N, chunk, tail};
+  if (!cache->keys.plans_fit(key)) {
+    cache->keys.drop_plans();
     cache->full.reset(new Plan(d, chunk, st));
     cache->part.reset(tail ? new Plan(d, tail, st) : nullptr);
     if (!cache->full->ok || (tail && !cache->part->ok)) {
@@ -861,12 +860,7 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
       cache->part.reset();
       return fft_fail(RGF_E_CUDA, "cuFFT plan");
     }
-    cache->dev = dev;
-    cache->nky = nky;
-    cache->nkz = nkz;
-    cache->N = d.N;
-    cache->chunk = chunk;
-    cache->tail = tail;
+    cache->keys.set_plans(key);
   }
   if (cufftSetStream(cache->full->h, st) != CUFFT_SUCCESS ||
       (cache->part && cufftSetStream(cache->part->h, st) != CUFFT_SUCCESS))
