@@ -765,11 +765,23 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
     if (col < lo || col > hi) continue;
     for (int64_t ix = 0; ix < nx; ix++) lines.push_back(i * nx + ix);
   }
+  if (lines.empty()) {
+    // nothing but zeros, in stream order: the one form of the call that a
+    // stream capture can hold
+    for (int a = 0; a < 3; a++) {
+      const cudaError_t e = cudaMemsetAsync(out[a], 0, sizeof(double2) * series * nx * nij, st);
+      if (e != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(e));
+    }
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(st, &cap);
+    if (e == cudaSuccess && cap == cudaStreamCaptureStatusNone) e = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? RGF_OK : fft_fail(RGF_E_CUDA, cudaGetErrorString(e));
+  }
   // elements outside the band are zero, as in the reference's zeroed buffers:
   // the runs of elements between banded ones, or everything where the runs
   // are many
   std::vector<std::pair<int64_t, int64_t>> gaps;
-  for (size_t q = 0; q <= lines.size(); q += nx) {
+  for (size_t q = 0; q <= lines.size(); q += nx) {   // lines come in runs of nx
     const int64_t from = q == 0 ? 0 : lines[q - nx] / nx + 1, to = q < lines.size() ? lines[q] / nx : nij;
     if (to > from) gaps.push_back({from, to});
   }
@@ -809,7 +821,6 @@ int run_fft_form(rgf_ctx* ctx, int mode, int64_t nm, int64_t nx, int64_t nen, in
   if (fe == cudaSuccess && gaps.size() == 1 && gaps[0].first == 0 && gaps[0].second == nij)
     fe = cudaStreamSynchronize(cache->fill);
   if (fe != cudaSuccess) return fft_fail(RGF_E_CUDA, cudaGetErrorString(fe));
-  if (lines.empty()) return RGF_OK;
   // the k-shift phase with the normalisation and dE folded in
   const double kPi = 3.14159265359;   // the reference's pi (src/green_rgf.f90:23)
   double2 dE;

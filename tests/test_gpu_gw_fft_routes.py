@@ -28,3 +28,28 @@ def test_fft_grids_on_both_routes(rgf, nky, nkz, nen):  # noqa: F811
     want += list(F.gw_self_energy_fft(*A[:3], *A[5:], nky, nkz, 1, 0, 1, 0.013))
     for g, w in zip(out, want):
         assert np.max(np.abs(g.cpu().numpy() - w)) <= TOL * np.max(np.abs(w))
+
+
+def test_slice_outside_the_band_can_be_captured(rgf):  # noqa: F811
+    """A slice without a banded element is zeroed in stream order and nothing
+    else, so the call can be part of a captured graph."""
+    import torch
+    A = [torch.ones(3, 2, 1, 8, dtype=torch.complex128, device="cuda") for _ in range(8)]
+    out = [torch.full_like(A[0], 7.0) for _ in range(6)]
+    grid = dict(nky=1, nkz=1, nm=4, ndiag=0, first_ij=2, dEn=0.01)
+    s = torch.cuda.Stream()
+    with rgf.Context(rgf.Options()) as ctx:
+        g = torch.cuda.CUDAGraph()
+        torch.cuda.synchronize()
+        with torch.cuda.graph(g, stream=s):
+            ctx.gw_polarization_fft(*A[:5], PL=out[0], PG=out[1], PR=out[2], spindeg=2.0, stream=s.cuda_stream, **grid)
+            ctx.gw_self_energy_fft(*A[:3], *A[5:], SL=out[3], SG=out[4], SR=out[5], stream=s.cuda_stream, **grid)
+        torch.cuda.synchronize()
+        assert all(torch.all(o == 7.0) for o in out)
+        g.replay()
+        torch.cuda.synchronize()
+        assert not any(torch.any(o != 0) for o in out)
+        out[0].fill_(7.0)
+        ctx.gw_polarization_fft(*A[:5], PL=out[0], PG=out[1], PR=out[2], spindeg=2.0, **grid)
+        torch.cuda.synchronize()
+        assert not torch.any(out[0] != 0)
