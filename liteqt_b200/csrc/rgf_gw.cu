@@ -272,13 +272,27 @@ __global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L
   for (int r = 0; r < R; r++) al[r] = ag[r] = ar[r] = T{};
 #pragma unroll
   for (int k = 0; k < 3 * R * V; k++) run[k][tid] = 0.0;
-  // Imaginary G, n = 0, diagonal element: P^R is a difference of equal sums
-  // (of equal products where k - q = k), i.e. zero or the rounding of the
-  // reference's order.  The thread that owns that output forms it in that
-  // order, product by product, beside the chains of multiply-adds.
-  const bool owner = IMAG && i == j && n0 + q0 <= 0 && n0 + q0 + R > 0;
+  // n = 0: with imaginary G that is symmetric in (i, j), diagonal elements
+  // among them, P^R is a difference of equal sums (of equal products where
+  // k - q = k), i.e. zero or the rounding of the reference's order.  It is
+  // formed in that order, product by product, beside the chains of
+  // multiply-adds: the threads form a chunk's terms, one each, and the thread
+  // that owns the output adds them up during the next chunk (P + Sigma at the
+  // sizes above 4.07 ms; formed and added by the owner alone 4.31).
+  static_assert(NT == kSteps, "a term a thread");
+  __shared__ T term[2][kSteps];
+  const bool zero_here = n0 <= 0 && n0 + kTile > 0;
+  const bool owner = zero_here && n0 + q0 <= 0 && n0 + q0 + R > 0;
   const int rz = (int)(-n0) - q0;
-  double pr0 = 0.0;
+  int chunk = 0;                                       // chunks done
+  T pr0{};
+  auto add_terms = [&](int c) {
+#pragma unroll 8
+    for (int u = 0; u < kSteps; u++) {
+      if constexpr (IMAG) pr0 += term[c & 1][u];
+      else pr0 = rgf::cadd(pr0, term[c & 1][u]);
+    }
+  };
   for (int64_t ik = 0; ik < nk; ik++) {
     const size_t xrow = (size_t)(line * nk + ik) * nen;
     const size_t vrow = (size_t)(line * nk + d.kd(ik, iq)) * nen, vrowT = (size_t)(lineT * nk + d.kd(ik, iq)) * nen;
@@ -296,6 +310,7 @@ __global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L
         vs[2][vpos<R>(t)] = in ? ((const T*)G.a[2])[vrow + vb + t] : T{};    // G^R
       }
       __syncthreads();
+      if (owner && chunk > 0) add_terms(chunk - 1);
       T w0[R], w1[R], w2[R];
 #pragma unroll
       for (int r = 1; r < R; r++) {
@@ -330,15 +345,20 @@ __global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L
         }
       }
       flush(run, reinterpret_cast<double*>(acc));
-      if constexpr (IMAG) {
-        if (owner)
-#pragma unroll 4
-          for (int u = 0; u < kSteps; u++) {
-            const int p = vpos<R>(u + kTile - 1 - q0 - rz);
-            pr0 += __dsub_rn(__dmul_rn(xs[0][u], vs[2][p]), __dmul_rn(xs[2][u], vs[1][p]));
-          }
+      if (zero_here) {
+        const int p = vpos<R>(tid + kTile - 1 + (int)n0);
+        if constexpr (IMAG)
+          term[chunk & 1][tid] = __dsub_rn(__dmul_rn(xs[0][tid], vs[2][p]), __dmul_rn(xs[2][tid], vs[1][p]));
+        else
+          term[chunk & 1][tid] =
+              rgf::cadd(rgf::cmul(xs[0][tid], rgf::cconj(vs[2][p])), rgf::cmul(xs[2][tid], vs[1][p]));
+        chunk++;
       }
     }
+  }
+  if (chunk > 0) {                                     // uniform over the CTA
+    __syncthreads();
+    if (owner) add_terms(chunk - 1);
   }
 #pragma unroll
   for (int r = 0; r < R; r++) {
@@ -347,7 +367,10 @@ __global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L
 #pragma unroll
     for (int v = 0; v < 3; v++) {
       double2 z = make_double2(run[(v * R + r) * V][tid], IMAG ? 0.0 : run[(v * R + r) * V + V - 1][tid]);
-      if (IMAG && v == 2 && owner && r == rz) z.x = pr0;
+      if (v == 2 && owner && r == rz) {
+        if constexpr (IMAG) z.x = pr0;
+        else z = pr0;
+      }
       ((double2*)out.a[v])[orow + nop] = rgf::cmul(z, scale);
     }
   }
