@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(GwCfg<IMAG>::TS) gw_s_kernel(GWDims d, Lines L
 #pragma unroll
     for (int v = 0; v < 3; v++) {
       const double2 z = make_double2(run[2 * (v * R + r)][tid], run[2 * (v * R + r) + 1][tid]);
-      ((double2*)out.a[v])[orow + e] = e == 0 ? rgf::czero() : rgf::cmul(z, scale);
+      ((double2*)out.a[v])[orow + e] = rgf::cmul(e == 0 ? rgf::czero() : z, scale);
     }
   }
 }
