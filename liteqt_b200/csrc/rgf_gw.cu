@@ -141,7 +141,6 @@ struct Lines {
 
 constexpr int kPackP = 64, kPackE = 32;   // elements x energies of a gather tile
 
-
 // Gathers three arrays into lines: the imaginary parts (IMAG) or the whole
 // values.  A CTA takes kPackP consecutive elements of the block x kPackE
 // energies of one (ix, k), so it reads contiguous runs and writes runs along
@@ -153,7 +152,7 @@ __global__ void __launch_bounds__(256) gw_pack_kernel(GWDims d, Lines L, Arrays3
   using T = std::conditional_t<IMAG, double, double2>;
   __shared__ T tile[kPackP][kPackE + 1];
   const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
-  const int64_t p0 = (int64_t)blockIdx.x * kPackP, e0 = (int64_t)blockIdx.y * kPackE;
+  const int64_t p0 = (int64_t)blockIdx.x * kPackP;
   const int64_t ik = blockIdx.z % nk, ixl = blockIdx.z / nk;
   auto band = [&](int64_t p, int64_t& slot) {
     if (p >= n2) return false;
@@ -165,28 +164,29 @@ __global__ void __launch_bounds__(256) gw_pack_kernel(GWDims d, Lines L, Arrays3
   const int lp = threadIdx.x % kPackP;
   const bool mine = band(p0 + lp, slot);
   if (!__syncthreads_or(mine)) return;
-  for (int v = 0; v < 3; v++) {
-    if (mine) {
-      bool bad = false;
-      for (int le = threadIdx.x / kPackP; le < kPackE; le += 256 / kPackP) {
-        const int64_t e = e0 + le;
-        if (e >= d.nen) break;
-        const double2 x = src.a[v][p0 + lp + n2 * ((L.ix0 + ixl) + d.nx * (e + d.nen * ik))];
-        bad |= !(isfinite(x.x) && isfinite(x.y));
-        if constexpr (IMAG) tile[lp][le] = x.y;
-        else tile[lp][le] = x;
+  for (int64_t e0 = (int64_t)blockIdx.y * kPackE; e0 < d.nen; e0 += (int64_t)gridDim.y * kPackE)
+    for (int v = 0; v < 3; v++) {
+      if (mine) {
+        bool bad = false;
+        for (int le = threadIdx.x / kPackP; le < kPackE; le += 256 / kPackP) {
+          const int64_t e = e0 + le;
+          if (e >= d.nen) break;
+          const double2 x = src.a[v][p0 + lp + n2 * ((L.ix0 + ixl) + d.nx * (e + d.nen * ik))];
+          bad |= !(isfinite(x.x) && isfinite(x.y));
+          if constexpr (IMAG) tile[lp][le] = x.y;
+          else tile[lp][le] = x;
+        }
+        if (bad) flags[ixl * L.slots + slot] = 1;
       }
-      if (bad) flags[ixl * L.slots + slot] = 1;
+      __syncthreads();
+      for (int q = threadIdx.x; q < kPackP * kPackE; q += 256) {
+        const int le = q % kPackE, pp = q / kPackE;
+        int64_t sl;
+        if (e0 + le < d.nen && band(p0 + pp, sl))
+          ((T*)dst.a[v])[((ixl * L.slots + sl) * nk + ik) * d.nen + e0 + le] = tile[pp][le];
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    for (int q = threadIdx.x; q < kPackP * kPackE; q += 256) {
-      const int le = q % kPackE, pp = q / kPackE;
-      int64_t sl;
-      if (e0 + le < d.nen && band(p0 + pp, sl))
-        ((T*)dst.a[v])[((ixl * L.slots + sl) * nk + ik) * d.nen + e0 + le] = tile[pp][le];
-    }
-    __syncthreads();
-  }
 }
 
 // ---------------------------------------------------------------- sums
@@ -486,26 +486,29 @@ constexpr int kOutP = 16, kOutE = 32;   // elements x energies of a scatter tile
 __global__ void __launch_bounds__(256) gw_p_scatter_kernel(GWDims d, Lines L, Lines3 P, Lines3 out) {
   __shared__ double2 tile[3][kOutP][kOutE + 1];
   const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
-  const int64_t p0 = (int64_t)blockIdx.x * kOutP, e0 = (int64_t)blockIdx.y * kOutE;
+  const int64_t p0 = (int64_t)blockIdx.x * kOutP;
   const int64_t iq = blockIdx.z % nk, ixl = blockIdx.z / nk;
   const int64_t lo = d.nen / 2 - 1 - d.nopmax, hi = d.nen / 2 - 1 + d.nopmax;
-  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
-    const int le = q % kOutE, lp = q / kOutE;
-    const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
-    const bool in = p < n2 && i - j <= L.nd && j - i <= L.nd && e >= lo && e <= hi;
+  for (int64_t e0 = (int64_t)blockIdx.y * kOutE; e0 < d.nen; e0 += (int64_t)gridDim.y * kOutE) {
+    for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+      const int le = q % kOutE, lp = q / kOutE;
+      const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
+      const bool in = p < n2 && i - j <= L.nd && j - i <= L.nd && e >= lo && e <= hi;
 #pragma unroll
-    for (int v = 0; v < 3; v++)
-      tile[v][lp][le] = in ? ((const double2*)P.a[v])[((ixl * L.slots + L.slot(i, j, d.nm)) * nk + iq) * d.nen + e]
-                           : rgf::czero();
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
-    const int lp = q % kOutP, le = q / kOutP;
-    const int64_t p = p0 + lp, e = e0 + le;
-    if (p >= n2 || e >= d.nen) continue;
-    const size_t o = (size_t)p + (size_t)n2 * ((L.ix0 + ixl) + (size_t)d.nx * (e + (size_t)d.nen * iq));
+      for (int v = 0; v < 3; v++)
+        tile[v][lp][le] = in ? ((const double2*)P.a[v])[((ixl * L.slots + L.slot(i, j, d.nm)) * nk + iq) * d.nen + e]
+                             : rgf::czero();
+    }
+    __syncthreads();
+    for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+      const int lp = q % kOutP, le = q / kOutP;
+      const int64_t p = p0 + lp, e = e0 + le;
+      if (p >= n2 || e >= d.nen) continue;
+      const size_t o = (size_t)p + (size_t)n2 * ((L.ix0 + ixl) + (size_t)d.nx * (e + (size_t)d.nen * iq));
 #pragma unroll
-    for (int v = 0; v < 3; v++) ((double2*)out.a[v])[o] = tile[v][lp][le];
+      for (int v = 0; v < 3; v++) ((double2*)out.a[v])[o] = tile[v][lp][le];
+    }
+    __syncthreads();
   }
 }
 
@@ -519,41 +522,44 @@ __global__ void __launch_bounds__(256) gw_s_scatter_kernel(GWDims d, Lines L, do
                                                            Lines3 S) {
   __shared__ double2 tile[3][kOutP][kOutE + 1];
   const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
-  const int64_t p0 = (int64_t)blockIdx.x * kOutP, e0 = (int64_t)blockIdx.y * kOutE;
+  const int64_t p0 = (int64_t)blockIdx.x * kOutP;
   const int64_t ik = blockIdx.z % nk, ixl = blockIdx.z / nk, ix = L.ix0 + ixl;
-  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
-    const int le = q % kOutE, lp = q / kOutE;
-    const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
-    double2 nl = rgf::czero(), ng = nl, nr = nl;
-    if (have && p < n2 && i - j <= L.nd && j - i <= L.nd && e < d.nen) {
-      const size_t a = (size_t)((ixl * L.slots + L.slot(i, j, d.nm)) * nk + ik) * d.nen + e;
-      const size_t b = (size_t)((ixl * L.slots + L.slot(j, i, d.nm)) * nk + ik) * d.nen + e;
-      const double2 *NL = (const double2*)N.a[0], *NG = (const double2*)N.a[1], *NR = (const double2*)N.a[2];
-      const double2 la = NL[a], lb = NL[b], ga = NG[a], gb = NG[b];
-      auto sym = [](double2 x, double2 y) { return make_double2((x.x + y.x) / 2.0, (x.y + y.y) / 2.0); };
-      nr = sym(make_double2(NR[a].x, (ga.y - la.y) / 2.0), make_double2(NR[b].x, (gb.y - lb.y) / 2.0));
-      nl = sym(la, lb);
-      ng = sym(ga, gb);
-    }
-    tile[0][lp][le] = nl;
-    tile[1][lp][le] = ng;
-    tile[2][lp][le] = nr;
-  }
-  __syncthreads();
   const bool all = d.nx < 5;                            // every block repeats block 3
   const int64_t d0 = all ? 0 : (ix == 2 ? 0 : ix), d1 = all ? d.nx - 1 : (ix == d.nx - 3 ? d.nx - 1 : ix);
-  for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
-    const int lp = q % kOutP, le = q / kOutP;
-    const int64_t p = p0 + lp, e = e0 + le;
-    if (p >= n2 || e >= d.nen) continue;
-    const size_t row = (size_t)d.nx * (e + (size_t)d.nen * ik);
-#pragma unroll
-    for (int v = 0; v < 3; v++) {
-      double2* A = (double2*)S.a[v];
-      const double2 s = A[(size_t)p + (size_t)n2 * (ix + row)];
-      const double2 r = rgf::cadd(s, rgf::cscale(rgf::csub(tile[v][lp][le], s), alpha));
-      for (int64_t b = d0; b <= d1; b++) A[(size_t)p + (size_t)n2 * (b + row)] = r;
+  for (int64_t e0 = (int64_t)blockIdx.y * kOutE; e0 < d.nen; e0 += (int64_t)gridDim.y * kOutE) {
+    for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+      const int le = q % kOutE, lp = q / kOutE;
+      const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
+      double2 nl = rgf::czero(), ng = nl, nr = nl;
+      if (have && p < n2 && i - j <= L.nd && j - i <= L.nd && e < d.nen) {
+        const size_t a = (size_t)((ixl * L.slots + L.slot(i, j, d.nm)) * nk + ik) * d.nen + e;
+        const size_t b = (size_t)((ixl * L.slots + L.slot(j, i, d.nm)) * nk + ik) * d.nen + e;
+        const double2 *NL = (const double2*)N.a[0], *NG = (const double2*)N.a[1], *NR = (const double2*)N.a[2];
+        const double2 la = NL[a], lb = NL[b], ga = NG[a], gb = NG[b];
+        auto sym = [](double2 x, double2 y) { return make_double2((x.x + y.x) / 2.0, (x.y + y.y) / 2.0); };
+        nr = sym(make_double2(NR[a].x, (ga.y - la.y) / 2.0), make_double2(NR[b].x, (gb.y - lb.y) / 2.0));
+        nl = sym(la, lb);
+        ng = sym(ga, gb);
+      }
+      tile[0][lp][le] = nl;
+      tile[1][lp][le] = ng;
+      tile[2][lp][le] = nr;
     }
+    __syncthreads();
+    for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
+      const int lp = q % kOutP, le = q / kOutP;
+      const int64_t p = p0 + lp, e = e0 + le;
+      if (p >= n2 || e >= d.nen) continue;
+      const size_t row = (size_t)d.nx * (e + (size_t)d.nen * ik);
+#pragma unroll
+      for (int v = 0; v < 3; v++) {
+        double2* A = (double2*)S.a[v];
+        const double2 s = A[(size_t)p + (size_t)n2 * (ix + row)];
+        const double2 r = rgf::cadd(s, rgf::cscale(rgf::csub(tile[v][lp][le], s), alpha));
+        for (int64_t b = d0; b <= d1; b++) A[(size_t)p + (size_t)n2 * (b + row)] = r;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -628,16 +634,20 @@ struct Workspace {
     char* p = base + len * before;
     return Lines3{{p, p + len * val, p + 2 * len * val}};
   }
+  // CTAs along energy: a tile each, or several where the grid's limit is met
+  static unsigned energy_tiles(const GWDims& d, int tile) {
+    return (unsigned)std::min<int64_t>((d.nen + tile - 1) / tile, 65535);
+  }
   void pack(const GWDims& d, const Lines& L, int64_t n, bool imag, const Arrays3& src, const Lines3& dst, int* fl,
             cudaStream_t st) const {
     cudaMemsetAsync(fl, 0, sizeof(int) * (size_t)n * slots, st);
-    const dim3 grid((unsigned)((d.nm * d.nm + kPackP - 1) / kPackP), (unsigned)((d.nen + kPackE - 1) / kPackE),
+    const dim3 grid((unsigned)((d.nm * d.nm + kPackP - 1) / kPackP), energy_tiles(d, kPackE),
                     (unsigned)(n * d.nky * d.nkz));
     if (imag) gw_pack_kernel<true><<<grid, 256, 0, st>>>(d, L, src, dst, fl);
     else gw_pack_kernel<false><<<grid, 256, 0, st>>>(d, L, src, dst, fl);
   }
   dim3 out_grid(const GWDims& d, int64_t n) const {
-    return dim3((unsigned)((d.nm * d.nm + kOutP - 1) / kOutP), (unsigned)((d.nen + kOutE - 1) / kOutE),
+    return dim3((unsigned)((d.nm * d.nm + kOutP - 1) / kOutP), energy_tiles(d, kOutE),
                 (unsigned)(n * d.nky * d.nkz));
   }
 };
