@@ -705,6 +705,9 @@ bool rgf::ctx_scratch(rgf_ctx* c, size_t bytes, void** p) {
   *p = c->scratch.p;
   return true;
 }
+void rgf::ctx_scratch_trim(rgf_ctx* c, size_t keep) {
+  if (c->scratch.bytes > keep) c->scratch.release();
+}
 void* rgf::ctx_ext_cache(rgf_ctx* c) { return c->ext_cache; }
 void rgf::ctx_set_ext_cache(rgf_ctx* c, void* cache, void (*free_fn)(void*)) {
   c->ext_cache = cache;

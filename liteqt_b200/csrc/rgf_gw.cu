@@ -17,6 +17,8 @@
 // Three passes: the banded elements are gathered into series contiguous in
 // energy, the sums run on those with R outputs a thread in registers, and a
 // scatter pass writes the caller's arrays (for S with the post-processing).
+// Where the device has no memory left for the series of one block, the sums
+// run on the caller's arrays as they are (gw_*_direct_kernel, no scratch).
 #include <algorithm>
 #include <cstdio>
 #include <type_traits>
@@ -77,7 +79,7 @@ __device__ __forceinline__ void cfma_to(double2& acc, double a, double2 b) {
 // One output of the polarization, summed in the reference's own order and
 // with its complex products (k, then E).  The tiled kernels use it for lines
 // that hold an infinity or a NaN, where leaving a term out is not the same as
-// adding a zero.
+// adding a zero, and the direct kernels for every element.
 __device__ __noinline__ void p_reference_sum(const GWDims& d, int imag_only, int64_t nop, int64_t i, int64_t j,
                                              int64_t ix, int64_t iq, Arrays3 G, double2 out[3]) {
   const double2 *GL = G.a[0], *GG = G.a[1], *GR = G.a[2];
@@ -512,11 +514,35 @@ __global__ void __launch_bounds__(256) gw_p_scatter_kernel(GWDims d, Lines L, Li
   }
 }
 
-// Sigma lines (N: S^<, S^>, S^R) -> the running self-energies: Sigma^R's
-// imaginary part from Sigma^> - Sigma^<, symmetrisation and mixing
-// (green_rgf.f90:3068-3085), then the edge-block copies (:3087-3092) in the
-// same pass: blocks 1, 2 repeat block 3 and blocks nx-1, nx block nx-2, so
-// only the blocks in between are summed and each writes its own copies.
+// New values of elements (i, j) and (j, i) -> what is mixed in at both:
+// Sigma^R's imaginary part from Sigma^> - Sigma^<, symmetrisation
+// (green_rgf.f90:3068-3081).
+__device__ __forceinline__ void s_post(const double2 (&a)[3], const double2 (&b)[3], double2 (&out)[3]) {
+  auto sym = [](double2 x, double2 y) { return make_double2((x.x + y.x) / 2.0, (x.y + y.y) / 2.0); };
+  out[0] = sym(a[0], b[0]);
+  out[1] = sym(a[1], b[1]);
+  out[2] = sym(make_double2(a[2].x, (a[1].y - a[0].y) / 2.0), make_double2(b[2].x, (b[1].y - b[0].y) / 2.0));
+}
+
+// Element p of block ix at (energy, k) = row / nx: mixing (:3083-3085) and the
+// edge-block copies (:3087-3092) in the same pass.  Blocks 1, 2 repeat block 3
+// and blocks nx-1, nx block nx-2, so only the blocks in between are summed and
+// each writes its own copies.
+__device__ __forceinline__ void s_mix(const GWDims& d, const Lines3& S, double alpha, int64_t p, int64_t ix, size_t row,
+                                      const double2 (&nv)[3]) {
+  const bool all = d.nx < 5;                            // every block repeats block 3
+  const int64_t d0 = all ? 0 : (ix == 2 ? 0 : ix), d1 = all ? d.nx - 1 : (ix == d.nx - 3 ? d.nx - 1 : ix);
+  const size_t n2 = (size_t)(d.nm * d.nm);
+#pragma unroll
+  for (int v = 0; v < 3; v++) {
+    double2* A = (double2*)S.a[v];
+    const double2 s = A[(size_t)p + n2 * (ix + row)];
+    const double2 r = rgf::cadd(s, rgf::cscale(rgf::csub(nv[v], s), alpha));
+    for (int64_t b = d0; b <= d1; b++) A[(size_t)p + n2 * (b + row)] = r;
+  }
+}
+
+// Sigma lines (N: S^<, S^>, S^R) -> the running self-energies (s_post, s_mix).
 // have = false: the window of offsets is empty and every new value is zero.
 __global__ void __launch_bounds__(256) gw_s_scatter_kernel(GWDims d, Lines L, double alpha, bool have, Lines3 N,
                                                            Lines3 S) {
@@ -524,42 +550,81 @@ __global__ void __launch_bounds__(256) gw_s_scatter_kernel(GWDims d, Lines L, do
   const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
   const int64_t p0 = (int64_t)blockIdx.x * kOutP;
   const int64_t ik = blockIdx.z % nk, ixl = blockIdx.z / nk, ix = L.ix0 + ixl;
-  const bool all = d.nx < 5;                            // every block repeats block 3
-  const int64_t d0 = all ? 0 : (ix == 2 ? 0 : ix), d1 = all ? d.nx - 1 : (ix == d.nx - 3 ? d.nx - 1 : ix);
   for (int64_t e0 = (int64_t)blockIdx.y * kOutE; e0 < d.nen; e0 += (int64_t)gridDim.y * kOutE) {
     for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
       const int le = q % kOutE, lp = q / kOutE;
       const int64_t p = p0 + lp, e = e0 + le, i = p % d.nm, j = p / d.nm;
-      double2 nl = rgf::czero(), ng = nl, nr = nl;
+      double2 nv[3] = {rgf::czero(), rgf::czero(), rgf::czero()};
       if (have && p < n2 && i - j <= L.nd && j - i <= L.nd && e < d.nen) {
         const size_t a = (size_t)((ixl * L.slots + L.slot(i, j, d.nm)) * nk + ik) * d.nen + e;
         const size_t b = (size_t)((ixl * L.slots + L.slot(j, i, d.nm)) * nk + ik) * d.nen + e;
-        const double2 *NL = (const double2*)N.a[0], *NG = (const double2*)N.a[1], *NR = (const double2*)N.a[2];
-        const double2 la = NL[a], lb = NL[b], ga = NG[a], gb = NG[b];
-        auto sym = [](double2 x, double2 y) { return make_double2((x.x + y.x) / 2.0, (x.y + y.y) / 2.0); };
-        nr = sym(make_double2(NR[a].x, (ga.y - la.y) / 2.0), make_double2(NR[b].x, (gb.y - lb.y) / 2.0));
-        nl = sym(la, lb);
-        ng = sym(ga, gb);
+        double2 na[3], nb[3];
+#pragma unroll
+        for (int v = 0; v < 3; v++) {
+          na[v] = ((const double2*)N.a[v])[a];
+          nb[v] = ((const double2*)N.a[v])[b];
+        }
+        s_post(na, nb, nv);
       }
-      tile[0][lp][le] = nl;
-      tile[1][lp][le] = ng;
-      tile[2][lp][le] = nr;
+#pragma unroll
+      for (int v = 0; v < 3; v++) tile[v][lp][le] = nv[v];
     }
     __syncthreads();
     for (int q = threadIdx.x; q < kOutP * kOutE; q += 256) {
       const int lp = q % kOutP, le = q / kOutP;
       const int64_t p = p0 + lp, e = e0 + le;
       if (p >= n2 || e >= d.nen) continue;
-      const size_t row = (size_t)d.nx * (e + (size_t)d.nen * ik);
-#pragma unroll
-      for (int v = 0; v < 3; v++) {
-        double2* A = (double2*)S.a[v];
-        const double2 s = A[(size_t)p + (size_t)n2 * (ix + row)];
-        const double2 r = rgf::cadd(s, rgf::cscale(rgf::csub(tile[v][lp][le], s), alpha));
-        for (int64_t b = d0; b <= d1; b++) A[(size_t)p + (size_t)n2 * (b + row)] = r;
-      }
+      const double2 nv[3] = {tile[0][lp][le], tile[1][lp][le], tile[2][lp][le]};
+      s_mix(d, S, alpha, p, ix, (size_t)d.nx * (e + (size_t)d.nen * ik), nv);
     }
     __syncthreads();
+  }
+}
+
+// ---------------------------------------------------------------- no scratch
+// The sums on the caller's arrays, one output a thread, in the reference's
+// order: for calls that find no memory for the series of one block.
+constexpr int kDirectThreads = 128;
+
+// grid: x = chunks of offsets, y = slot of the band, z = k-point + nk * block;
+// the rest of the arrays was zeroed
+__global__ void __launch_bounds__(kDirectThreads) gw_p_direct_kernel(GWDims d, Lines L, double2 scale, int imag_only,
+                                                                     Arrays3 G, Lines3 out) {
+  const int64_t nk = d.nky * d.nkz, iq = blockIdx.z % nk, ix = blockIdx.z / nk;
+  const int64_t i = blockIdx.y % d.nm, j = i - L.nd + blockIdx.y / d.nm;
+  const int64_t nop = -d.nopmax + (int64_t)blockIdx.x * kDirectThreads + threadIdx.x;
+  if (j < 0 || j >= d.nm || nop > d.nopmax) return;
+  double2 a[3];
+  p_reference_sum(d, imag_only, nop, i, j, ix, iq, G, a);
+  for (int v = 0; v < 3; v++) ((double2*)out.a[v])[d.at(i, j, ix, nop + d.nen / 2 - 1, iq)] = rgf::cmul(a[v], scale);
+}
+
+// grid: x = chunks of energies, y = elements of the block (strided), z =
+// k-point + nk * (block - ix0); a thread owns elements (i, j) and (j, i)
+__global__ void __launch_bounds__(kDirectThreads) gw_s_direct_kernel(GWDims d, Lines L, double2 scale, double alpha,
+                                                                     bool have, int imag_only, Arrays3 G, Arrays3 W,
+                                                                     Lines3 S) {
+  const int64_t nk = d.nky * d.nkz, ik = blockIdx.z % nk, ix = L.ix0 + blockIdx.z / nk;
+  const int64_t e = (int64_t)blockIdx.x * kDirectThreads + threadIdx.x;
+  if (e >= d.nen) return;
+  const size_t row = (size_t)d.nx * (e + (size_t)d.nen * ik);
+  for (int64_t p = blockIdx.y; p < d.nm * d.nm; p += gridDim.y) {
+    const int64_t i = p % d.nm, j = p / d.nm;
+    if (i > j) continue;
+    double2 nv[3] = {rgf::czero(), rgf::czero(), rgf::czero()};
+    if (have && j - i <= L.nd) {
+      double2 a[3], b[3];
+      s_reference_sum(d, imag_only, e + 1, i, j, ix, ik, G, W, a);
+      s_reference_sum(d, imag_only, e + 1, j, i, ix, ik, G, W, b);
+#pragma unroll
+      for (int v = 0; v < 3; v++) {
+        a[v] = rgf::cmul(a[v], scale);
+        b[v] = rgf::cmul(b[v], scale);
+      }
+      s_post(a, b, nv);
+    }
+    s_mix(d, S, alpha, p, ix, row, nv);
+    if (i != j) s_mix(d, S, alpha, j + d.nm * i, ix, row, nv);
   }
 }
 
@@ -602,30 +667,37 @@ int gw_fail(int code, const char* msg) {
   return code;
 }
 
-// Scratch of one call (the context's, kept between calls): the lines of as
-// many blocks ix as fit kWorkBytes, at least one, and a flag per line.  The
-// calls return with their stream drained, so the next one may reuse it.
+// Scratch of one call (the context's, kept between calls up to kWorkBytes):
+// the lines of as many blocks ix as fit kWorkBytes, at least one, and a flag
+// per line.  The calls return with their stream drained, so the next one may
+// reuse it.
 struct Workspace {
-  static constexpr size_t kWorkBytes = size_t(2) << 30;
+  static constexpr size_t kWorkBytes = size_t(256) << 20;
+  rgf_ctx* ctx = nullptr;
   int64_t nd = 0, slots = 0, nix = 0;
   size_t per_line = 0;
-  char* base = nullptr;
+  char* base = nullptr;      // NULL: no memory for one block's lines
   int* flags = nullptr;
 
+  ~Workspace() {
+    if (ctx) rgf::ctx_scratch_trim(ctx, kWorkBytes);
+  }
   // bytes_per_value: of all the lines arrays together
-  int open(rgf_ctx* ctx, const GWDims& d, int64_t ix0, int64_t ix1, size_t bytes_per_value, int nflags) {
+  void open(rgf_ctx* c, const GWDims& d, int64_t ix0, int64_t ix1, size_t bytes_per_value, int nflags) {
+    ctx = c;
     nd = std::min(d.ndiag, d.nm - 1);
     slots = d.nm * (2 * nd + 1);
     per_line = (size_t)d.nky * d.nkz * d.nen;
-    const size_t per_ix = (size_t)slots * per_line * bytes_per_value;
-    nix = std::max<int64_t>(1, std::min<int64_t>(ix1 - ix0, (int64_t)(kWorkBytes / per_ix)));
-    const size_t lines = (per_ix * nix + 255) & ~size_t(255);
+    const size_t per_ix = ((size_t)slots * per_line * bytes_per_value + 255) & ~size_t(255);
+    const size_t flag_bytes = sizeof(int) * (size_t)nflags * slots;
+    nix = std::max<int64_t>(1, std::min<int64_t>(ix1 - ix0, (int64_t)(kWorkBytes / (per_ix + flag_bytes))));
     void* p = nullptr;
-    if (!rgf::ctx_scratch(ctx, lines + sizeof(int) * (size_t)nflags * nix * slots, &p))
-      return gw_fail(RGF_E_NOMEM, "device scratch for the convolutions");
+    if (!rgf::ctx_scratch(ctx, (per_ix + flag_bytes) * nix, &p)) {
+      nix = 1;
+      if (!rgf::ctx_scratch(ctx, per_ix + flag_bytes, &p)) return;
+    }
     base = (char*)p;
-    flags = (int*)(base + lines);
-    return RGF_OK;
+    flags = (int*)(base + per_ix * nix);
   }
   // three lines arrays of `val`-byte values for n blocks, after `before` bytes
   // per value (the 16-byte ones first, which keeps them aligned)
@@ -677,6 +749,7 @@ extern "C" int rgf_gw_polarization(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nk = nky * nkz;
   const size_t bytes = sizeof(rgf_c16) * (size_t)nm * nm * nx * nen * nk;
+  Workspace ws;
   View gl, gg, gr, pl, pg, pr;
   cudaError_t e = gl.open((void*)G_lesser, bytes, true, false, st);
   if (e == cudaSuccess) e = gg.open((void*)G_greater, bytes, true, false, st);
@@ -694,9 +767,14 @@ extern "C" int rgf_gw_polarization(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t
     const Lines3 out{{pl.dev, pg.dev, pr.dev}};
     const size_t val = imag_only ? sizeof(double) : sizeof(double2);
     const int64_t tile = imag_only ? GwCfg<true>::TILE : GwCfg<false>::TILE;
-    Workspace ws;
-    if ((rc = ws.open(ctx, d, 0, nx, 3 * val + 3 * sizeof(double2), 1)) != RGF_OK) return rc;
-    for (int64_t ix0 = 0; ix0 < nx; ix0 += ws.nix) {
+    ws.open(ctx, d, 0, nx, 3 * val + 3 * sizeof(double2), 1);
+    if (!ws.base) {
+      for (View* v : {&pl, &pg, &pr}) cudaMemsetAsync(v->dev, 0, bytes, st);
+      const dim3 grid((unsigned)((2 * d.nopmax + kDirectThreads) / kDirectThreads), (unsigned)ws.slots,
+                      (unsigned)(nx * nk));
+      gw_p_direct_kernel<<<grid, kDirectThreads, 0, st>>>(d, Lines{ws.nd, ws.slots, 0}, scale, imag_only, G, out);
+    }
+    for (int64_t ix0 = 0; ws.base && ix0 < nx; ix0 += ws.nix) {
       const int64_t n = std::min(ws.nix, nx - ix0);
       const Lines L{ws.nd, ws.slots, ix0};
       const Lines3 pp = ws.take(sizeof(double2), n, 0), gp = ws.take(val, n, 3 * sizeof(double2));
@@ -729,6 +807,7 @@ extern "C" int rgf_gw_self_energy(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t 
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t nk = nky * nkz;
   const size_t bytes = sizeof(rgf_c16) * (size_t)nm * nm * nx * nen * nk;
+  Workspace ws;
   View gl, gg, gr, wl, wg, wr, sl, sg, sr;
   cudaError_t e = gl.open((void*)G_lesser, bytes, true, false, st);
   if (e == cudaSuccess) e = gg.open((void*)G_greater, bytes, true, false, st);
@@ -753,9 +832,14 @@ extern "C" int rgf_gw_self_energy(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t 
   const int64_t first = 2, last = nx < 5 ? 2 : nx - 3;
   const size_t val = imag_only ? sizeof(double) : sizeof(double2);
   const int64_t tile = imag_only ? GwCfg<true>::TILE : GwCfg<false>::TILE;
-  Workspace ws;
-  if ((rc = ws.open(ctx, d, first, last + 1, 3 * val + 6 * sizeof(double2), 2)) != RGF_OK) return rc;
-  for (int64_t ix0 = first; ix0 <= last; ix0 += ws.nix) {
+  ws.open(ctx, d, first, last + 1, 3 * val + 6 * sizeof(double2), 2);
+  if (!ws.base) {
+    const dim3 grid((unsigned)((nen + kDirectThreads - 1) / kDirectThreads),
+                    (unsigned)std::min<int64_t>(nm * nm, 65535), (unsigned)((last + 1 - first) * nk));
+    gw_s_direct_kernel<<<grid, kDirectThreads, 0, st>>>(d, Lines{ws.nd, ws.slots, first}, scale, alpha_mix, have,
+                                                        imag_only, G, W, S);
+  }
+  for (int64_t ix0 = first; ws.base && ix0 <= last; ix0 += ws.nix) {
     const int64_t n = std::min(ws.nix, last + 1 - ix0);
     const Lines L{ws.nd, ws.slots, ix0};
     const Lines3 wp = ws.take(sizeof(double2), n, 0), np = ws.take(sizeof(double2), n, 3 * sizeof(double2)),

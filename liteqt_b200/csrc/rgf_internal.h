@@ -167,6 +167,8 @@ cudaError_t launch_block_fp64_inv(int nb, const double2* X, double2* Xi, int64_t
 // drained: at least `bytes`, kept until the context is destroyed or a call
 // needs more.  false: out of memory.
 bool ctx_scratch(rgf_ctx* c, size_t bytes, void** p);
+// Gives the scratch back if it is larger than `keep` (stream drained).
+void ctx_scratch_trim(rgf_ctx* c, size_t keep);
 // Per-context state owned by another module (one slot): a pointer and the
 // function that frees it when the context is destroyed.
 void* ctx_ext_cache(rgf_ctx* c);
