@@ -36,6 +36,7 @@
 // energy fastest, ik = ikz + nkz (iky) (0-based).  nen must be even.
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -671,7 +672,9 @@ int run_own(FftCache* cache, int dev, int mode, const Dims& d, int logm, const s
   }
   chunk = chunk < 1 ? 1 : (chunk > nl ? nl : chunk);
   if (chunk > 65535) chunk = 65535;                             // grid y
-  const int64_t ctas = (int64_t)sms * L.per_sm;
+  // scratch for the CTAs that work, not more than a chunk keeps busy: short
+  // calls need little memory
+  const int64_t ctas = std::min((int64_t)sms * L.per_sm, (chunk * d.nk + L.group - 1) / L.group);
   const size_t scr = (size_t)ctas * L.group * 3 * M;
   int rc = reserve_scratch(cache, dev, sizeof(double2) * (per_line * chunk + scr + ph.size()) + sizeof(int64_t) * nl, st);
   if (rc) return rc;

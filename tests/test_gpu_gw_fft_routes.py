@@ -53,3 +53,34 @@ def test_slice_outside_the_band_can_be_captured(rgf):  # noqa: F811
         ctx.gw_polarization_fft(*A[:5], PL=out[0], PG=out[1], PR=out[2], spindeg=2.0, **grid)
         torch.cuda.synchronize()
         assert not torch.any(out[0] != 0)
+
+
+def test_short_call_close_to_the_memory_limit(rgf):  # noqa: F811
+    """Four series of 64 energies with 24 MB left on the device."""
+    import torch
+    rng = np.random.default_rng(1)
+    A = [rng.normal(size=(1, 2, 2, 64)) + 1j * rng.normal(size=(1, 2, 2, 64)) for _ in range(5)]
+    D = [torch.from_numpy(a).cuda() for a in A]
+    out = [torch.zeros_like(D[0]) for _ in range(3)]
+
+    def run():
+        with rgf.Context(rgf.Options()) as ctx:
+            ctx.gw_polarization_fft(*D, PL=out[0], PG=out[1], PR=out[2], nky=1, nkz=2, nm=1, ndiag=0, first_ij=1,
+                                    dEn=0.01, spindeg=1.0)
+    run()       # loads the kernels
+    for o in out:
+        o.zero_()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    for unit in (1 << 30, 16 << 20, 2 << 20):
+        while torch.cuda.mem_get_info()[0] > (24 << 20) + unit:
+            held.append(torch.cuda.caching_allocator_alloc(unit))
+    try:
+        run()
+    finally:
+        for p in held:
+            torch.cuda.caching_allocator_delete(p)
+        torch.cuda.empty_cache()
+    for g, w in zip(out, F.gw_polarization_fft(*A, 1, 2, 1, 0, 1, 0.01, 1.0)):
+        assert np.max(np.abs(g.cpu().numpy() - w)) <= TOL * np.max(np.abs(w))
