@@ -22,6 +22,7 @@
 #include <thread>
 #include <vector>
 
+#include "rgf_inflight.h"
 #include "rgf_internal.h"
 
 #if defined(__x86_64__) && defined(__SSE2__)
@@ -671,6 +672,7 @@ struct rgf_ctx {
   rgf_stats stats;
   int8_t variant[kVariantSlots];  // kernel variant per block size (defaults; rgf_autotune may override)
   int8_t ctas[kVariantSlots];     // resident CTAs per SM per block size, 0 = as many as fit
+  InFlight::Ticket pipe_ticket[2];   // of the pipelined calls, until their pipe_solved
   DevBuf scratch;                 // ctx_scratch, on CUDA device scratch_dev
   int scratch_dev = -1;
   void* ext_cache = nullptr;      // per-context state of other modules (the FFT form's plans)
@@ -780,6 +782,7 @@ extern "C" int rgf_ctx_destroy(rgf_ctx* c) {
   if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
   if (c->ext_cache_free) c->ext_cache_free(c->ext_cache);
   for (int b = 0; b < 2; b++) {
+    c->pipe_ticket[b].reset();
     c->pipe_stage[b].release();
     c->pipe_dinfo[b].release();
     if (c->pipe_free[b]) cudaEventDestroy(c->pipe_free[b]);
@@ -1067,8 +1070,17 @@ static int launch_ctas_per_sm(const rgf_ctx* c, size_t smem, uint64_t nb_mask) {
 //   nb = 256,  18 energies:  402 /  227 /  128 /  120*   148 energies:  436 /  405*
 // So: no clusters up to nb = 32; otherwise the largest that leaves every CTA
 // an SM of its own; two CTAs an SM from nb = 192 on, and from nb = 80 on where
-// there would be no cluster otherwise.
-static SolverShape solver_shape(const rgf_ctx* c, size_t smem, uint64_t nb_mask, int64_t n_tasks) {
+// there would be no cluster otherwise.  `others`: tasks of other calls at work
+// on the GPU, which need SMs too.  Threads with a context each, nx = 20,
+// energies/s by single CTAs / by clusters as if alone / by this rule (twelve
+// calls a thread; the first ones, made before the others are seen, cost the
+// few percent):
+//   nb =  64, 12 energies a call: 4 threads 3796 / 1691 / 4393, 8 threads 7458 / 1820 / 6875
+//   nb = 128, 12 energies a call: 4 threads  616 /  595 /  942, 8 threads 1196 /  637 / 1341
+//   nb = 128,  1 energy a call:  16 threads  109 /  352 /  354
+// room: the tasks, others included, up to which the geometry holds.
+static SolverShape solver_shape(const rgf_ctx* c, size_t smem, uint64_t nb_mask, int64_t n_tasks, int64_t others,
+                                int64_t* room = nullptr) {
   SolverShape s;
   const int resident = c->sm_count * launch_ctas_per_sm(c, smem, nb_mask);
   s.groups = (int)std::min<int64_t>(resident, n_tasks);
@@ -1083,24 +1095,47 @@ static SolverShape solver_shape(const rgf_ctx* c, size_t smem, uint64_t nb_mask,
       if (v == KV_GENERIC11 || v == KV_GENERIC12 || v == KV_GENERIC22) return s;
       nb = 8 * i;
     }
-  if (nb <= 32 || 2 * n_tasks > resident) return s;
+  const int64_t all = n_tasks + others;
+  if (nb <= 32 || 2 * all > resident) return s;
   smem = std::max(smem, variant_smem(KV_TILED, nb));
   const size_t alone = std::max<size_t>(smem, 120 * 1024);   // more than two CTAs of an SM can have
   auto fits = [&](int k, size_t bytes, int ctas) {
-    return n_tasks * k <= ctas && solver_max_clusters(bytes, k) >= n_tasks;
+    if (all * k > ctas) return false;
+    const int64_t most = std::min<int64_t>(ctas / k, solver_max_clusters(bytes, k));
+    if (most < all) return false;
+    s.cluster = k;
+    s.smem = bytes;
+    if (room) *room = most;
+    return true;
   };
-  for (int k = 8; k > 1 && s.cluster == 1; k /= 2)
-    if (fits(k, alone, c->sm_count)) {
-      s.cluster = k;
-      s.smem = alone;
-    }
+  for (int k = 8; k > 1; k /= 2)
+    if (fits(k, alone, c->sm_count)) break;
   if (nb >= 192 || (nb >= 80 && s.cluster == 1))
     for (int k = 8; k > s.cluster; k /= 2)
-      if (fits(k, smem, resident)) {
-        s.cluster = k;
-        s.smem = smem;
-      }
+      if (fits(k, smem, resident)) break;
   return s;
+}
+
+// The process's solver calls in flight (never destroyed: threads of the host
+// program may outlive static objects).
+static InFlight& in_flight() {
+  static InFlight* b = new InFlight();
+  return *b;
+}
+// Tasks that other streams' calls have on the context's GPU.  Launches of
+// different streams run beside one another up to the count of the device's
+// hardware queues: 8, or what CUDA_DEVICE_MAX_CONNECTIONS sets.
+static int64_t others_in_flight(const rgf_ctx* c, cudaStream_t st) {
+  static const int queues = [] {
+    const char* e = std::getenv("CUDA_DEVICE_MAX_CONNECTIONS");
+    const int n = e ? std::atoi(e) : 0;
+    return n >= 1 && n <= 32 ? n : 8;
+  }();
+  return in_flight().others(c->device, st, queues, [](void* ev) {
+    const cudaError_t e = cudaEventQuery((cudaEvent_t)ev);
+    if (e == cudaErrorNotReady) cudaGetLastError();
+    return e != cudaErrorNotReady;
+  });
 }
 
 // Checks a task list; RGF_OK or the error.
@@ -1292,7 +1327,8 @@ extern "C" int rgf_solve_batch(rgf_ctx* c, const rgf_device* devices, int32_t n_
   const LaunchShape shape = launch_shape(c, devices, tasks, n_tasks);
   const std::vector<int32_t>& order = shape.order;
   int64_t slot = shape.slot;
-  const SolverShape geo = solver_shape(c, shape.smem, shape.nb_mask, n_tasks);
+  InFlight::Ticket ticket(in_flight(), c->device, st, n_tasks);
+  const SolverShape geo = solver_shape(c, shape.smem, shape.nb_mask, n_tasks, others_in_flight(c, st));
   int grid = geo.groups;
   if (mixed) {
     int64_t nx_max = 2;
@@ -1355,6 +1391,8 @@ extern "C" int rgf_solve_batch(rgf_ctx* c, const rgf_device* devices, int32_t n_
     // ---- outputs back: the copier queues them as the blocks are written;
     // the call returns now
     RGF_CUDA(cudaEventRecord(c->pipe_solved[pb], st));
+    ticket.until(c->pipe_solved[pb]);
+    c->pipe_ticket[pb] = std::move(ticket);
     PipeJob j;
     j.slot = pb;
     j.prog = c->pipe_prog[pb];
@@ -1549,7 +1587,8 @@ extern "C" int rgf_adjoint_energies(rgf_ctx* c, const rgf_device* v, int64_t nen
   RGF_CUDA(cudaMemsetAsync(c->info.p, 0, sizeof(DInfo) * nen, st));
   RGF_CUDA(cudaMemsetAsync(c->queue.p, 0, sizeof(int32_t), st));
   const size_t smem = variant_smem(c->variant[nm / 8], (int)nm);
-  const SolverShape geo = solver_shape(c, smem, 1ull << (nm / 8), nen);
+  InFlight::Ticket ticket(in_flight(), c->device, st, nen);
+  const SolverShape geo = solver_shape(c, smem, 1ull << (nm / 8), nen, others_in_flight(c, st));
   const int64_t slot = slot_elems_for(nm, nx);
   if ((rc = c->work.reserve(sizeof(double2) * (size_t)slot * geo.groups))) return rc;
   KParams p;
@@ -1924,11 +1963,20 @@ struct rgf_plan {
   int64_t n_tasks = 0;
   std::vector<int> task_nb;
   DevBuf work, tasks, devs, info, queue;
-  cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
+  // the launch, and where that takes clusters the launch of single CTAs for
+  // when other calls' tasks leave them no room
+  cudaGraph_t graph[2] = {nullptr, nullptr};
+  cudaGraphExec_t exec[2] = {nullptr, nullptr};
+  int64_t room = 0;              // solver_shape's
+  InFlight::Ticket ticket;       // of the last execution, until `done`
+  cudaEvent_t done = nullptr;
   ~rgf_plan() {
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    ticket.reset();
+    if (done) cudaEventDestroy(done);
+    for (int k = 0; k < 2; k++) {
+      if (exec[k]) cudaGraphExecDestroy(exec[k]);
+      if (graph[k]) cudaGraphDestroy(graph[k]);
+    }
     work.release();
     tasks.release();
     devs.release();
@@ -1995,7 +2043,7 @@ extern "C" int rgf_plan_create(rgf_ctx* c, const rgf_device* devices, int32_t n_
     pl->task_nb[t] = (int)devices[k.device].nm;
   }
   const LaunchShape shape = launch_shape(c, devices, tasks, n_tasks);
-  const SolverShape geo = solver_shape(c, shape.smem, shape.nb_mask, n_tasks);
+  const SolverShape geo = solver_shape(c, shape.smem, shape.nb_mask, n_tasks, 0, &pl->room);
   if ((rc = pl->work.reserve(sizeof(double2) * (size_t)shape.slot * geo.groups))) return rc;
   if ((rc = pl->devs.reserve(sizeof(DDev) * n_devices))) return rc;
   if ((rc = pl->tasks.reserve(sizeof(DTask) * n_tasks + sizeof(int32_t) * n_tasks))) return rc;
@@ -2015,18 +2063,27 @@ extern "C" int rgf_plan_create(rgf_ctx* c, const rgf_device* devices, int32_t n_
   p.work = (double2*)pl->work.p;
   p.slot_elems = shape.slot;
   p.info = (DInfo*)pl->info.p;
+  RGF_CUDA(cudaEventCreateWithFlags(&pl->done, cudaEventDisableTiming));
   solver_blocks_per_sm(geo.smem);  // sets the kernel's shared-memory limit before the capture
   cudaStream_t cs = nullptr;
   RGF_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-  cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-  if (e == cudaSuccess) {
-    cudaError_t e1 = cudaMemsetAsync(pl->queue.p, 0, sizeof(int32_t), cs);
-    cudaError_t e2 = cudaMemsetAsync(pl->info.p, 0, sizeof(DInfo) * n_tasks, cs);
-    cudaError_t e3 = launch_solver(p, geo, cs, false);
-    e = cudaStreamEndCapture(cs, &pl->graph);
-    if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < (geo.cluster > 1 ? 2 : 1) && e == cudaSuccess; k++) {
+    SolverShape g = geo;
+    if (k == 1) {                  // as many CTAs as the clusters, so the same work slots
+      g.cluster = 1;
+      g.smem = shape.smem;
+    }
+    e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
+    if (e == cudaSuccess) {
+      cudaError_t e1 = cudaMemsetAsync(pl->queue.p, 0, sizeof(int32_t), cs);
+      cudaError_t e2 = cudaMemsetAsync(pl->info.p, 0, sizeof(DInfo) * n_tasks, cs);
+      cudaError_t e3 = launch_solver(p, g, cs, false);
+      e = cudaStreamEndCapture(cs, &pl->graph[k]);
+      if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
+    }
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&pl->exec[k], pl->graph[k], 0);
   }
-  if (e == cudaSuccess) e = cudaGraphInstantiate(&pl->exec, pl->graph, 0);
   cudaStreamDestroy(cs);
   if (e != cudaSuccess) return fail(RGF_E_CUDA, "plan capture failed: %s", cudaGetErrorString(e));
   *out = pl.release();
@@ -2038,10 +2095,25 @@ extern "C" int rgf_plan_execute(rgf_plan* pl, rgf_task_info* info, void* stream_
   rgf_ctx* c = pl->ctx;
   RGF_CUDA(cudaSetDevice(c->device));
   cudaStream_t st = stream_ ? (cudaStream_t)stream_ : c->stream;
+  // a caller's capture holds the plan's own geometry and no queries
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  RGF_CUDA(cudaStreamIsCapturing(st, &cap));
+  const bool live = cap == cudaStreamCaptureStatusNone;
+  InFlight::Ticket ticket;
+  int k = 0;
+  if (live) {
+    ticket = InFlight::Ticket(in_flight(), c->device, st, pl->n_tasks);
+    if (pl->exec[1] && pl->n_tasks + others_in_flight(c, st) > pl->room) k = 1;
+  }
   RGF_CUDA(cudaEventRecord(c->ev0, st));
-  RGF_CUDA(cudaGraphLaunch(pl->exec, st));
+  RGF_CUDA(cudaGraphLaunch(pl->exec[k], st));
   RGF_CUDA(cudaEventRecord(c->ev1, st));
   c->stats.launches++;
+  if (live && !info) {
+    RGF_CUDA(cudaEventRecord(pl->done, st));
+    ticket.until(pl->done);
+    pl->ticket = std::move(ticket);
+  }
   if (!info) return RGF_OK;
   std::vector<DInfo> h(pl->n_tasks);
   RGF_CUDA(cudaStreamSynchronize(st));   // see rgf_solve_batch: no pageable copy behind a running kernel
@@ -2252,7 +2324,8 @@ extern "C" int rgf_w_solve_batch(rgf_ctx* c, const rgf_w_device* devices, int32_
     nb_mask |= 1ull << (v.nm / 8);
   }
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return cost[a] > cost[b]; });
-  const SolverShape geo = solver_shape(c, smem, nb_mask, n_tasks);
+  InFlight::Ticket ticket(in_flight(), c->device, st, n_tasks);
+  const SolverShape geo = solver_shape(c, smem, nb_mask, n_tasks, others_in_flight(c, st));
   if ((rc = c->work.reserve(sizeof(double2) * (size_t)slot * geo.groups))) return rc;
   if ((rc = c->devs.reserve(sizeof(DDev) * n_devices))) return rc;
   if ((rc = c->tasks.reserve(sizeof(DWTask) * n_tasks + sizeof(int32_t) * n_tasks))) return rc;
