@@ -151,6 +151,10 @@ struct TiledOps {
       if (grp.size == 1) return gj_invert_panel<64, NC, 0>(grp, n, X, dst, dst2, inv, dyn + (size_t)n * n);
       return gj_invert_tiled<64, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
     }
+    if constexpr (NC == 0) {
+      if (n <= 128) return gj_invert_rank8<128>(grp, n, X, Rt, dst, dst2, dyn, inv);
+      return gj_invert_rank8<256>(grp, n, X, Rt, dst, dst2, dyn, inv);
+    }
     if (n <= 128) return gj_invert_tiled<128, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
     return gj_invert_tiled<256, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
   }

@@ -285,16 +285,18 @@ __device__ __noinline__ int gj_invert_reg(G grp, int n, const double2* X, double
 //   (3) every thread updates its own elements, x_ij - f_i r_j.
 // The pivot key is the high word of the bit pattern of |re|+|im| (monotonic
 // for non-negative doubles), so entries within 2^-20 of each other count as
-// equal and the first row among them is taken; rows above k have key 0, NaN
-// entries key 1 (never chosen unless the whole column is NaN, then row k as
-// the scalar search), exact zeros key 2 and every other entry a larger key.
+// equal and the first row among them is taken; EXACT: ties of the high word
+// go by the low word (the block sizes whose unblocked search compared all
+// bits).  Rows above k have key 0, NaN entries key 1 (never chosen unless the
+// whole column is NaN, then row k as the scalar search), exact zeros key 2
+// and every other entry a larger key.
 // The per-element arithmetic is that of the unblocked elimination.  scr:
 // 2 NB + 6 KB + 2 NB/32 complex values of scratch, double-buffered by column
 // parity so one column's readers never race the next column's writers.
 // Returns with the sub-block written back to the panel and a barrier passed;
 // s.singular is set on a zero pivot.
 // n <= NB rows; threads of rows from n on carry zeros that are never pivots.
-template <int NB>
+template <int NB, bool EXACT = false>
 __device__ __forceinline__ void gj_subblock(int n, int LD, double2* panel, int PW, int p0, int sb0, double2* scr,
                                             int16_t* rmap, SmemInv& s) {
   constexpr int KB = 8;
@@ -309,6 +311,7 @@ __device__ __forceinline__ void gj_subblock(int n, int LD, double2* panel, int P
   double2* pinvw = rk + 2 * KB;  // [2][WPC] per-warp winner's reciprocal
   unsigned* pk = reinterpret_cast<unsigned*>(pinvw + 2 * WPC);  // [2][WPC] keys
   int* pi = reinterpret_cast<int*>(pk + 2 * WPC);               // [2][WPC] rows
+  unsigned* pl = reinterpret_cast<unsigned*>(pi + 2 * WPC);     // [2][WPC] low words (EXACT)
   double2 x[CPT];
 #pragma unroll
   for (int m = 0; m < CPT; m++) x[m] = i < n ? panel[i + (sb0 + h * CPT + m) * LD] : czero();
@@ -323,13 +326,21 @@ __device__ __forceinline__ void gj_subblock(int n, int LD, double2* panel, int P
       unsigned key = 0u;
       if (i >= k && i < n) {
         const unsigned hi = (unsigned)((unsigned long long)__double_as_longlong(av) >> 32);
-        key = !(av == av) ? 1u : (av == 0.0 ? 2u : (hi > 1u ? hi : 1u) + 2u);
+        key = !(av == av) ? 1u : (av == 0.0 ? 2u : EXACT ? hi + 3u : (hi > 1u ? hi : 1u) + 2u);
       }
       const double2 pv = crecip(v);
       const unsigned kmax = __reduce_max_sync(0xffffffffu, key);
-      const unsigned imin = __reduce_min_sync(0xffffffffu, key == kmax ? (unsigned)i : 0xffffffffu);
+      bool top = key == kmax;
+      unsigned lmax = 0u;
+      if constexpr (EXACT) {
+        const unsigned lo = top ? (unsigned)__double_as_longlong(av) : 0u;
+        lmax = __reduce_max_sync(0xffffffffu, kmax > 2u ? lo : 0u);
+        top = top && (kmax <= 2u || lo == lmax);
+      }
+      const unsigned imin = __reduce_min_sync(0xffffffffu, top ? (unsigned)i : 0xffffffffu);
       if ((unsigned)i == imin) {
         const int w = warp - hc * WPC;
+        if constexpr (EXACT) pl[par * WPC + w] = lmax;
         pk[par * WPC + w] = kmax;
         pi[par * WPC + w] = i;
         pinvw[par * WPC + w] = pv;
@@ -337,12 +348,19 @@ __device__ __forceinline__ void gj_subblock(int n, int LD, double2* panel, int P
     }
     __syncthreads();
     unsigned key = pk[par * WPC];
+    unsigned low = EXACT ? pl[par * WPC] : 0u;
     int q = pi[par * WPC], wq = 0;
 #pragma unroll
     for (int w = 1; w < WPC; w++) {
       const unsigned ek = pk[par * WPC + w];
       const int ei = pi[par * WPC + w];
-      if (ek > key || (ek == key && ei < q)) { key = ek; q = ei; wq = w; }
+      bool more = ek > key || (ek == key && ei < q);
+      if constexpr (EXACT) {
+        const unsigned el = pl[par * WPC + w];
+        more = ek > key || (ek == key && (el > low || (el == low && ei < q)));
+        if (more) low = el;
+      }
+      if (more) { key = ek; q = ei; wq = w; }
     }
     // largest |re|+|im| zero: flagged, and the caller discards the block
     if (key == 2u && tid == 0) s.singular = 1;

@@ -7,8 +7,10 @@
 // follow the block size, dealt to the CTAs of the group.  Shared tiles are
 // k-major with a row pitch of 66 complex values (conflict-free fragments).
 //
-// Inverse: as rgf_staged.cuh's, the panel's own columns left out of the
-// update; up to 72 rows one panel holds the whole block.
+// Inverse: for nb = 64, 128, 256 as rgf_staged.cuh's, in panels, the panel's
+// own columns left out of the update.  For the other sizes, whose unblocked
+// elimination had a smaller error than panels have, 8 columns at a time
+// (gj_invert_rank8).
 #pragma once
 #include "rgf_staged.cuh"
 
@@ -29,14 +31,16 @@ __host__ __device__ constexpr int padded_rows(int n) { return n <= 64 ? 64 : (n 
 // Shared scratch of the elimination (complex values): pivot column twice,
 // pivot rows and candidates; the rank-8 update's 8 x PW pivot rows share it.
 __host__ __device__ constexpr int sub_scratch(int nbp) { return 2 * nbp + 48 + nbp / 16; }
-// Panel width of the blocked inverse: the whole block up to 72 rows, else as
-// wide as the shared memory holds at a pitch of n + 2 (which makes the rank-8
-// updates' fragment reads of 4 columns x 2 rows hit 8 distinct 16-byte bank
-// groups) beside the scratch, at most 48.
-__host__ __device__ constexpr int panel_width(int n) {
-  const int sub = sub_scratch(padded_rows(n)), room = (kSmemValues - (sub > 320 ? sub : 320)) / (n + 2) / 8 * 8;
-  return n <= 72 ? n : (room < 48 ? room : 48);
+// Panel width of the blocked inverse: nb = 64 whole; 48 columns at nb = 128;
+// 16 at nb = 256 (24 fit, 1 % faster, but with an error against 64 bits 1.04
+// to 1.17 times that of 16).  Pitch n + 2, which makes the rank-8 updates'
+// fragment reads of 4 columns x 2 rows hit 8 distinct 16-byte bank groups.
+__host__ __device__ constexpr int panel_width(int n) { return n <= 64 ? n : (n <= 128 ? 48 : 16); }
+constexpr bool panel_fits(int n) {
+  return (n + 2) * panel_width(n) + (n <= 64 ? 8 * (n - 8) : 320) <= kSmemValues &&
+         (n + 2) * panel_width(n) + sub_scratch(padded_rows(n)) <= kSmemValues;
 }
+static_assert(panel_fits(64) && panel_fits(128) && panel_fits(256), "panel");
 
 struct AllCols {
   __device__ __forceinline__ int operator()(int j) const { return j; }
@@ -387,6 +391,118 @@ __device__ __noinline__ int gj_invert_tiled(const Group& grp, int n_, double2* X
           }
         },
         rmap + p0, [&](int j) { return j < p0 ? j : j + PW; });
+    grp.sync();
+    double2* t = cur;
+    cur = nxt;
+    nxt = t;
+  }
+  const int sing = s.singular;
+  __syncthreads();
+  return sing ? zero_inverse(grp, n, dst, dst2) : 0;
+}
+
+// Gauss-Jordan inverse of the n x n block X0 (global memory, ld n, destroyed)
+// for the block sizes without a panel form, result into dst (and dst2); X1: a
+// second global block.  Eight columns at a time: eliminated in registers
+// (gj_subblock), then all other columns get them as one rank-8 update, its
+// four real products per half summed apart and added to the element once.
+// Longer sums round more often: at nb = 80 .. 248 the inverse's error against
+// 64 bits is 1.2 to 1.6 times the unblocked elimination's with panels of 48,
+// 0.7 to 1.0 times with this form (solves at nb = 80 .. 200: 1.2 to 1.7 and
+// 1.00 to 1.08 times).  Rows are gathered through the map of the eight
+// columns' interchanges while the two blocks alternate, as in
+// gj_invert_tiled.  Bound by the elimination's column chain and by the round
+// trips of n / 8 passes over the block through L2, so a warp has four output
+// subtiles' loads in flight (200 energies at nb = 104, nx = 30: 152 ms; panels
+// through the tiled product 151 ms at 48 columns, 195 ms at 8; unblocked, with
+// the register-direct product, 217 ms).  In a group every CTA eliminates its
+// own copy of the eight columns; the subtiles are shared.
+// Returns 1 (and zeros dst) on a zero pivot.
+template <int NB>
+__device__ __noinline__ int gj_invert_rank8(const Group& grp, int n, double2* X0, double2* X1, double2* dst,
+                                            double2* dst2, double2* smem, SmemInv& s) {
+  constexpr int KB = 8, kRow = 12;                   // pivot rows' pitch: 4 x 2 fragments on distinct banks
+  static_assert(KB * (NB + 2) + kRow * NB + sub_scratch(NB) <= kSmemValues, "shared memory");
+  const int LD = n + 2, r8 = n >> 3, tiles = r8 * (r8 - 1);
+  double2* panel = smem;                             // [8][LD]
+  double2* rows = panel + KB * LD;                   // [n][kRow] pivot rows of the other columns
+  double2* scr = rows + kRow * n;
+  int16_t* rmap = s.rmap;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t4 = lane & 3;
+  const int step = kWarps * grp.size;
+  double2* cur = X0;
+  double2* nxt = X1;
+  if (tid == 0) s.singular = 0;
+  for (int p0 = 0; p0 < n; p0 += KB) {
+    for (int e = tid; e < KB * n; e += kThreads) {
+      const int jj = e / n, i = e - jj * n;
+      cp_async16(panel + i + jj * LD, cur + (size_t)p0 * n + e);
+    }
+    cp_async_commit();
+    for (int i = tid; i < n; i += kThreads) rmap[i] = (int16_t)i;
+    cp_async_wait<0>();
+    __syncthreads();
+    gj_subblock<NB, true>(n, LD, panel, KB, p0, 0, scr, rmap, s);
+    if (s.singular) break;
+    // the last step writes the inverse itself: column c goes to coldst[c]
+    const bool last = p0 + KB >= n;
+    if (last) undo_interchanges(n, s);
+    auto put = [&](int i, int j, double2 v) {
+      if (last) {
+        const size_t o = i + (size_t)s.coldst[j] * n;
+        dst[o] = v;
+        if (dst2) dst2[o] = v;
+      } else {
+        nxt[i + (size_t)j * n] = v;
+      }
+    };
+    for (int e = tid; e < KB * n; e += kThreads) {
+      const int t = e & (KB - 1), j = e >> 3;
+      if (j < p0 || j >= p0 + KB) cp_async16(rows + t + j * kRow, cur + rmap[p0 + t] + (size_t)j * n);
+    }
+    cp_async_commit();
+    for (int e = tid + kThreads * grp.rank; e < KB * n; e += kThreads * grp.size) {
+      const int jj = e / n, i = e - jj * n;
+      put(i, p0 + jj, panel[i + jj * LD]);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    constexpr int U = 4;
+    for (int t0 = warp + kWarps * grp.rank; t0 < tiles; t0 += U * step) {
+      double2 x[U][2];
+      int row[U], col[U];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int q = t0 + u * step, b = q / r8;
+        row[u] = 8 * (q - b * r8);
+        col[u] = 8 * (8 * b < p0 ? b : b + 1);
+        x[u][0] = x[u][1] = czero();
+        if (q < tiles && row[u] != p0) {
+          const double2* at = cur + rmap[row[u] + g] + (size_t)(col[u] + 2 * t4) * n;
+          x[u][0] = at[0];
+          x[u][1] = at[n];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        if (t0 + u * step >= tiles) break;
+        double rr[2][2] = {}, ii[2][2] = {}, ri[2][2] = {}, ir[2][2] = {};   // [4 columns of the panel][output]
+#pragma unroll
+        for (int ks = 0; ks < 2; ks++) {
+          const double2 a = panel[row[u] + g + (4 * ks + t4) * LD];
+          const double2 b = rows[4 * ks + t4 + (col[u] + g) * kRow];
+          dmma884(rr[ks][0], rr[ks][1], a.x, b.x);
+          dmma884(ri[ks][0], ri[ks][1], a.x, b.y);
+          dmma884(ii[ks][0], ii[ks][1], a.y, b.y);
+          dmma884(ir[ks][0], ir[ks][1], a.y, b.x);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+          put(row[u] + g, col[u] + 2 * t4 + c,
+              make_double2(x[u][c].x + ((rr[0][c] - ii[0][c]) + (rr[1][c] - ii[1][c])),
+                           x[u][c].y + ((ri[0][c] + ir[0][c]) + (ri[1][c] + ir[1][c]))));
+      }
+    }
     grp.sync();
     double2* t = cur;
     cur = nxt;
