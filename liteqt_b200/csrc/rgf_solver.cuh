@@ -114,20 +114,19 @@ struct StagedOps {
     // slower); larger: panels.  The same arithmetic as TiledOps, so a task's
     // results do not depend on how many CTAs share it.
     if constexpr (NB == 32) return gj_invert_reg(grp, NB, X, dst, dst2, inv, dyn + (size_t)NB * NB);
-    else if constexpr (NB == 64) return gj_invert_panel<NB, NB, 0>(Group{}, NB, X, dst, dst2, inv, dyn + (size_t)NB * NB);
+    else if constexpr (NB == 64) return gj_invert_panel<NB, 0>(Group{}, X, dst, dst2, inv, dyn + (size_t)NB * NB);
     else if constexpr (NB == 128) return gj_invert_blocked<NB>(X, Rt, dst, dst2, dyn, dyn, inv);
-    else return gj_invert_tiled<NB, NB>(Group{}, NB, X, Rt, dst, dst2, dyn, inv);
+    else return gj_invert_tiled<NB>(Group{}, X, Rt, dst, dst2, dyn, inv);
   }
   // >= NB complex values of shared memory free between block operations
   __device__ double2* scratch() const { return dyn; }
 };
 
-// The tiled operations of rgf_tiled.cuh: any nb that is a multiple of 8 (NC =
-// 0), and nb = NC where a cluster shares a task (the size at compile time is
-// worth 1.2x there: nb = 128 on 8 CTAs 35 against 42 ms for 12 energies).  Up
-// to nb = 64 the matrix to invert is assembled in shared memory (a product is
-// one tile there, so nothing loads stages over it), unless several CTAs
-// assemble it.
+// The tiled operations of rgf_tiled.cuh: nb from 80 on that are multiples of 8
+// and have no staged form (NC = 0), and nb = NC where a cluster shares a task
+// (the size at compile time is worth 1.2x there: nb = 128 on 8 CTAs 35 against
+// 42 ms for 12 energies).  The matrix to invert is assembled in the slot: the
+// CTAs of a cluster share it, and larger blocks do not fit shared memory.
 template <int NC>
 struct TiledOps {
   static constexpr bool kMixed = false, kGroup = true;
@@ -137,26 +136,22 @@ struct TiledOps {
   double2* X;
   double2* Rt;
   Group grp;
-  __device__ TiledOps(SmemInv& i, double2* dyn_, double2* slot_inv, double2* slot_rt, int n, Group g)
-      : inv(i), dyn(dyn_), X((NC ? NC : n) <= 64 && g.size == 1 ? dyn_ : slot_inv), Rt(slot_rt), grp(g) {}
+  __device__ TiledOps(SmemInv& i, double2* dyn_, double2* slot_inv, double2* slot_rt, int, Group g)
+      : inv(i), dyn(dyn_), X(slot_inv), Rt(slot_rt), grp(g) {}
   template <class Epi>
   __device__ void gemm(int n_, const double2* A, bool cA, const double2* B, bool cB, Epi&& epi) {
     const int n = NC ? NC : n_;
     gemm_tiles(grp, n, n, n, A, n, cA, B, n, cB, dyn, NoInit{}, epi, nullptr, AllCols{});
   }
-  __device__ int invert(int n_, double2* dst, double2* dst2) {
-    const int n = NC ? NC : n_;
-    if (n <= 32) return gj_invert_reg(grp, n, X, dst, dst2, inv, dyn + 32 * 32);
-    if (n <= 64) {
-      if (grp.size == 1) return gj_invert_panel<64, NC, 0>(grp, n, X, dst, dst2, inv, dyn + (size_t)n * n);
-      return gj_invert_tiled<64, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
-    }
+  __device__ int invert(int n, double2* dst, double2* dst2) {
     if constexpr (NC == 0) {
       if (n <= 128) return gj_invert_rank8<128>(grp, n, X, Rt, dst, dst2, dyn, inv);
       return gj_invert_rank8<256>(grp, n, X, Rt, dst, dst2, dyn, inv);
+    } else if constexpr (NC == 32) {
+      return gj_invert_reg(grp, NC, X, dst, dst2, inv, dyn);
+    } else {
+      return gj_invert_tiled<NC>(grp, X, Rt, dst, dst2, dyn, inv);
     }
-    if (n <= 128) return gj_invert_tiled<128, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
-    return gj_invert_tiled<256, NC>(grp, n, X, Rt, dst, dst2, dyn, inv);
   }
   // >= nb complex values of shared memory free between block operations
   __device__ double2* scratch() const { return dyn; }

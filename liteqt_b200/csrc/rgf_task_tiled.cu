@@ -1,5 +1,5 @@
-// rgf_task_tiled.cu -- RGF task function for any nb (multiple of 8): tiled GEMM and Gauss-Jordan with the block size
-// at run time, by one CTA or a cluster.
+// rgf_task_tiled.cu -- RGF task function for nb from 80 on (multiples of 8 without a staged form): tiled GEMM and
+// Gauss-Jordan with the block size at run time, by one CTA or a cluster.
 #include "rgf_solver.cuh"
 #include "rgf_tasks.h"
 

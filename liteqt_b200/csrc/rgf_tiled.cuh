@@ -2,6 +2,10 @@
 // the size known at run time, by one CTA or by the CTAs of a thread-block
 // cluster together (Group).
 //
+// Used for the block sizes from 80 on without a staged form (size at run time)
+// and, with the size at compile time, for nb = 32, 64, 128 and 256 where a
+// cluster shares a task.
+//
 // GEMM: as rgf_staged.cuh's (K in chunks of 16 through three cp.async stages,
 // 8 warps of DMMA), but the output is cut into tiles of at most 64 x 64 that
 // follow the block size, dealt to the CTAs of the group.  Shared tiles are
@@ -267,7 +271,7 @@ __device__ __forceinline__ int zero_inverse(const Group& grp, int n, double2* ds
   return 1;
 }
 
-// Gauss-Jordan inverse (partial pivoting) of the n x n block that `panel`
+// Gauss-Jordan inverse (partial pivoting) of the block of n = NB that `panel`
 // (shared memory, pitch n + PAD) holds whole: 8-column sub-blocks eliminated with
 // their elements in registers (gj_subblock) and the other columns updated by
 // rank-8 DMMA products (panel_rank8_update).  Then dst[:, j] =
@@ -275,10 +279,10 @@ __device__ __forceinline__ int zero_inverse(const Group& grp, int n, double2* ds
 // of a group eliminates its own copy and writes its share.  scr: shared
 // scratch of max(8 (n - 8), sub_scratch(NB)) complex values.  Returns 1 (and
 // zeros dst) on a zero pivot.
-template <int NB, int NC, int PAD>
-__device__ __noinline__ int gj_invert_panel(const Group& grp, int n_, double2* panel, double2* dst,
-                                               double2* dst2, SmemInv& s, double2* scr) {
-  const int n = NC ? NC : n_, LD = n + PAD;
+template <int NB, int PAD>
+__device__ __noinline__ int gj_invert_panel(const Group& grp, double2* panel, double2* dst, double2* dst2, SmemInv& s,
+                                            double2* scr) {
+  constexpr int n = NB, LD = n + PAD;
   if (threadIdx.x == 0) s.singular = 0;
   for (int i = threadIdx.x; i < n; i += kThreads) s.rmap[i] = (int16_t)i;
   __syncthreads();
@@ -301,7 +305,7 @@ __device__ __noinline__ int gj_invert_panel(const Group& grp, int n_, double2* p
   return 0;
 }
 
-// Blocked Gauss-Jordan inverse of the n x n block X0 (global memory, ld n,
+// Blocked Gauss-Jordan inverse of the block X0 of n = NB (global memory, ld n,
 // destroyed), result into dst (and dst2).  X1: a second global block.
 // The row interchanges of a panel are never applied in place: the panel's
 // update reads the permuted rows of the current matrix (row gather in the
@@ -314,11 +318,10 @@ __device__ __noinline__ int gj_invert_panel(const Group& grp, int n_, double2* p
 // eliminates its own copy of the panel (the elimination is a serial chain,
 // which a broadcast would only lengthen) and the update's tiles are shared.
 // Returns 1 (and zeros dst) on a zero pivot.
-template <int NB, int NC>
-__device__ __noinline__ int gj_invert_tiled(const Group& grp, int n_, double2* X0, double2* X1, double2* dst, double2* dst2,
-                                 double2* smem, SmemInv& s) {
-  const int n = NC ? NC : n_;
-  const int PWM = panel_width(n), LD = n + 2;
+template <int NB>
+__device__ __noinline__ int gj_invert_tiled(const Group& grp, double2* X0, double2* X1, double2* dst, double2* dst2,
+                                            double2* smem, SmemInv& s) {
+  constexpr int n = NB, PWM = panel_width(n), LD = n + 2;
   double2* panel = smem;
   double2* scr = panel + LD * PWM;
   int16_t* rmap = s.rmap;
@@ -333,9 +336,9 @@ __device__ __noinline__ int gj_invert_tiled(const Group& grp, int n_, double2* X
     cp_async_wait<0>();
     __syncthreads();
   };
-  if (PWM >= n) {
+  if constexpr (PWM >= n) {
     load_panel(X0, n);
-    return gj_invert_panel<NB, NC, 2>(grp, n, panel, dst, dst2, s, scr);
+    return gj_invert_panel<NB, 2>(grp, panel, dst, dst2, s, scr);
   }
   double2* cur = X0;
   double2* nxt = X1;
