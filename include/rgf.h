@@ -207,7 +207,9 @@ RGF_API int rgf_solve_batch(rgf_ctx* ctx, const rgf_device* devices, int32_t n_d
  * Every array the devices and tasks reference must be device memory and stay
  * valid while the plan exists; their contents may change between executions
  * (they are read when the graph runs), the energies and addresses may not.
- * The plan keeps the context's options and kernel choices of creation time. */
+ * The plan keeps the context's options and kernel choices of creation time; a
+ * plan of few tasks spreads each over a cluster of CTAs unless solver calls on
+ * other streams leave too few SMs when it is executed (the same results). */
 typedef struct rgf_plan rgf_plan;
 RGF_API int rgf_plan_create(rgf_ctx* ctx, const rgf_device* devices, int32_t n_devices,
                             const rgf_task* tasks, int64_t n_tasks, rgf_plan** plan);
@@ -361,6 +363,9 @@ RGF_API int rgf_green_rgf_calc_w(rgf_ctx* ctx, const int64_t* NBC, const int64_t
  * symmetrisation (:3070-3081), mixing into Sigma_*_gw with alpha_mix
  * (:3083-3085) and the copies of blocks 3 / nx-2 into the two edge blocks of
  * each side (:3087-3092); Sigma_*_gw are updated in place (nx >= 3).
+ * Both gather the band into device scratch, of which the context keeps up to
+ * 256 MB between calls; a call that finds no memory for one block's share
+ * runs without scratch, several times slower.
  * Error text: rgf_gw_last_error(). */
 RGF_API int rgf_gw_polarization(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t nen, int64_t nky,
                                 int64_t nkz, int64_t ndiag, double dE, double spindeg,
@@ -391,12 +396,15 @@ RGF_API const char* rgf_gw_last_error(void);
  *   rgf_gw_self_energy_fft: Sigma^< = sum_q conv(G^<_kd, W^<_q), Sigma^>
  *     likewise, Sigma^R = conv(G^<, W^R) + conv(G^R, W^<) + conv(G^R, W^R),
  *     times i dEn/(2 pi)/nk, then Sigma^R = Re + i Im(Sigma^> - Sigma^<)/2.
- * The transforms are cuFFT's, in chunks of (i,j, ix) lines within at most
- * 4 GB of device scratch (RGF_GW_FFT_CHUNK sets the lines per chunk); the
- * context keeps the scratch and the cuFFT plans of the last shape between
- * calls and frees them in rgf_ctx_destroy.
- * Stream-ordered on `stream`; returns when the results are written.  Error
- * text: rgf_gw_fft_last_error(). */
+ * Up to nen = 4096 the transforms are the library's own where they are the
+ * faster form (k-grids of 1, 2 or 4 points an axis always, others by their
+ * size), in chunks of (i,j, ix) lines within about 1 GB of device scratch;
+ * otherwise cuFFT's, within 4 GB (RGF_GW_FFT_CHUNK sets the lines per chunk).
+ * The context keeps the scratch, its tables and the cuFFT plans of the last
+ * shape between calls and frees them in rgf_ctx_destroy.
+ * Stream-ordered on `stream`; returns when the results are written (a slice
+ * without a banded element, on a capturing stream: when its zeros are
+ * captured).  Error text: rgf_gw_fft_last_error(). */
 RGF_API int rgf_gw_polarization_fft(rgf_ctx* ctx, int64_t nm, int64_t nx, int64_t nen, int64_t nky,
                                     int64_t nkz, int64_t ndiag, int64_t nij, int64_t first_ij, double dEn,
                                     double spindeg, const rgf_c16* G_lesser, const rgf_c16* G_greater,
