@@ -1064,10 +1064,10 @@ static int launch_ctas_per_sm(const rgf_ctx* c, size_t smem, uint64_t nb_mask) {
 // time (measured on 1 B200, nx = 10, G^R, G^<, G^>, ms with clusters of 1 / 2 /
 // 4 / 8, * = two CTAs on an SM):
 //   nb =  32,   1 energy:    1.9 /  2.7 /  2.7 /  2.7    cluster barriers cost more than the products
-//   nb =  64,  37 energies:  9.5 /  7.9 /  9.1*
-//   nb =  96,  37 energies: 42.9 / 26.4 / 25.5*          120 energies: 48.8 / 39.1*
-//   nb = 128,  18 energies: 55.0 / 34.9 / 23.1 / 25.7*   148 energies: 61.3 / 60.2*
-//   nb = 256,  18 energies:  402 /  227 /  128 /  120*   148 energies:  436 /  405*
+//   nb =  64,  37 energies:  9.9 /  8.3 /  9.6*
+//   nb =  96,  37 energies: 46.8 / 29.0 / 26.1*          120 energies: 52.2 / 41.6*
+//   nb = 128,  18 energies: 57.9 / 36.5 / 24.3           148 energies: 64.9 / 64.0*
+//   nb = 256,  18 energies:  445 /  248 /  137 /  124*   148 energies:  518 /  437*
 // So: no clusters up to nb = 32; otherwise the largest that leaves every CTA
 // an SM of its own; two CTAs an SM from nb = 192 on, and from nb = 80 on where
 // there would be no cluster otherwise.  `others`: tasks of other calls at work

@@ -205,9 +205,9 @@ __global__ void __launch_bounds__(256) gw_pack_kernel(GWDims d, Lines L, Arrays3
 // finite here (other lines take the reference sum), so values outside a
 // series are zeros in shared memory instead of conditions in the loop.
 // Measured (1 B200, 1965 MHz) at nk = 4, nen = 512, nx = 10, nm = 16,
-// ndiag = 3, imaginary G: P 7.7 -> 1.75 ms, Sigma 12.6 -> 1.75 ms (complex
+// ndiag = 3, imaginary G: P 7.7 -> 1.79 ms, Sigma 12.6 -> 1.80 ms (complex
 // products on values staged whole, one output a thread, before), i.e. 14 and
-// 17 TFLOP/s of real multiply-adds; gathers 0.17 ms, scatters 0.31 ms.
+// 16 TFLOP/s of real multiply-adds; gathers 0.31 ms, scatters 0.22 ms.
 constexpr int kSteps = 64;
 
 template <bool IMAG>
