@@ -205,9 +205,9 @@ __global__ void __launch_bounds__(256) gw_pack_kernel(GWDims d, Lines L, Arrays3
 // finite here (other lines take the reference sum), so values outside a
 // series are zeros in shared memory instead of conditions in the loop.
 // Measured (1 B200, 1965 MHz) at nk = 4, nen = 512, nx = 10, nm = 16,
-// ndiag = 3, imaginary G: P 7.7 -> 1.79 ms, Sigma 12.6 -> 1.80 ms (complex
-// products on values staged whole, one output a thread, before), i.e. 14 and
-// 16 TFLOP/s of real multiply-adds; gathers 0.31 ms, scatters 0.22 ms.
+// ndiag = 3, imaginary G: P 7.7 -> 1.64 ms, Sigma 12.6 -> 1.80 ms (complex
+// products on values staged whole, one output a thread, before), i.e. 15 and
+// 16 TFLOP/s of real multiply-adds; gathers 0.32 ms, scatters 0.18 ms.
 constexpr int kSteps = 64;
 
 template <bool IMAG>
@@ -216,6 +216,7 @@ struct GwCfg {
   static constexpr int RP = IMAG ? 8 : 4;              // outputs a thread, polarization
   static constexpr int RS = 4;                         // self-energy
   static constexpr int TP = TILE / RP, TS = TILE / RS;  // threads
+  static constexpr int kPerSm = IMAG ? 5 : 6;          // CTAs of gw_p_kernel an SM: bounds its registers
 };
 
 template <int R>
@@ -241,7 +242,7 @@ __device__ __forceinline__ void flush(double (&run)[N][NT], double* part) {
 // With purely imaginary G every product is one real multiply-add.  G: the
 // lines of G^<, G^>, G^R; out: lines [line][q][energy of n].
 template <bool IMAG>
-__global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L, double2 scale, int imag_only,
+__global__ void __launch_bounds__(GwCfg<IMAG>::TP, GwCfg<IMAG>::kPerSm) gw_p_kernel(GWDims d, Lines L, double2 scale, int imag_only,
                                                                Arrays3 src, Lines3 G, Lines3 out,
                                                                const int* __restrict__ flags) {
   using T = std::conditional_t<IMAG, double, double2>;
@@ -280,7 +281,7 @@ __global__ void __launch_bounds__(GwCfg<IMAG>::TP) gw_p_kernel(GWDims d, Lines L
   // formed in that order, product by product, beside the chains of
   // multiply-adds: the threads form a chunk's terms, one each, and the thread
   // that owns the output adds them up during the next chunk (P + Sigma at the
-  // sizes above 4.07 ms; formed and added by the owner alone 4.31).
+  // sizes above 4.0 ms; formed and added by the owner alone 4.3).
   static_assert(NT == kSteps, "a term a thread");
   __shared__ T term[2][kSteps];
   const bool zero_here = n0 <= 0 && n0 + kTile > 0;
@@ -544,7 +545,7 @@ __device__ __forceinline__ void s_mix(const GWDims& d, const Lines3& S, double a
 
 // Sigma lines (N: S^<, S^>, S^R) -> the running self-energies (s_post, s_mix).
 // have = false: the window of offsets is empty and every new value is zero.
-__global__ void __launch_bounds__(256) gw_s_scatter_kernel(GWDims d, Lines L, double alpha, bool have, Lines3 N,
+__global__ void __launch_bounds__(256, 3) gw_s_scatter_kernel(GWDims d, Lines L, double alpha, bool have, Lines3 N,
                                                            Lines3 S) {
   __shared__ double2 tile[3][kOutP][kOutE + 1];
   const int64_t n2 = d.nm * d.nm, nk = d.nky * d.nkz;
